@@ -6,8 +6,8 @@
 
 #include <math.h>
 
-#include "cycle.cuh"
 #include "engine.h"
+#include "patch.cuh"
 
 namespace dgpu {
 
@@ -23,15 +23,18 @@ __device__ __forceinline__ double apply_cell(const Lvl64& L, const double* __res
     return v;
 }
 
-// Per-CTA layout for one side-n problem. Global arena (L2-resident while the
-// CTA works on the problem): the FP64 hierarchy (e, nf, d, id per level,
-// wb/sb boundary vectors), the five FP64 CG vectors b, r, p, Ap, z, the
-// cycle's own coefficient copies and iterate/right-hand side for the large
-// levels, and the scratch used once per problem to build the dense tail.
-// Shared memory: level 0's cycle data when all of it fits in `sbudget` bytes,
-// then the dense tail operator, then the cycle's data for as many coarse
-// levels as fit. Level 0 of an FP64 cycle works directly on r (right-hand
-// side) and z (iterate).
+// Per-CTA layout for one side-n problem, every level in the padded layout of
+// patch.cuh. Global arena (L2-resident while the CTA works on the problem):
+// the FP64 hierarchy (e, nf, d, id per level, wb/sb boundary vectors), the
+// FP64 CG vectors r, p, Ap and u, the cycle's arrays that are not in shared
+// memory, and the scratch used once per problem to build the dense tail. The
+// level-0 vectors of an FP64 cycle are CG's own: r (right-hand side) and z
+// (iterate).
+//
+// Shared memory, up to `sbudget` bytes: the dense tail operator, then the
+// cycle's arrays level by level from the coarsest (a visit of level l moves
+// ~4^-l of level 0's bytes and happens 2^l times per W-cycle, so a byte of a
+// coarse level is read more often), in a level the arrays most read first.
 //
 // Dense tail: the levels from tl (the first level of side <= kBlockTailSide,
 // when that is not level 0) down implement the fixed map "x = 0, then gamma
@@ -41,39 +44,46 @@ __device__ __forceinline__ double apply_cell(const Lvl64& L, const double* __res
 // 2^k levels below. Same operator as the recursion, to rounding.
 // Shared by host sizing and device carving (gbase/sbase == null: size only).
 constexpr int kBlockTailSide = 8;
+constexpr int kBlockLevels = 20;  // sides below 2^17: more than the int cell index allows
 
 struct BlockLayout {
     size_t global_bytes, smem_bytes;
-    int nlev, ls;
+    int nlev;
 };
 
 template <class T>
 struct BlockViews {
-    Lvl64 h[kMaxLevels];        // FP64 hierarchy
-    Lvl<T> lv[kMaxLevels];      // the cycle's levels
-    Lvl<T> lm[kMaxLevels];      // tail construction: the tail levels with N right-hand sides, in the
+    Lvl64 h[kBlockLevels];      // FP64 hierarchy; .n is the side, arrays padded
+    PLvl<T> lv[kBlockLevels];   // the cycle's levels
+    PLvl<T> lm[kBlockLevels];   // tail construction: the tail levels with N right-hand sides, in the
                                 // cycle's precision (FP32 copies of the coefficients for the mixed form)
-    double* cg[5];              // b, r, p, Ap, z
-    T* tail;                    // dense tail operator (ntail x ntail), or null
-    int nlev, tl, ntail;
+    double *r, *p, *ap, *u;     // CG vectors (padded)
+    T* tail;                    // dense tail operator (ntail rows of tail_pitch), or null
+    int nlev, tl, ntail;        // ntail: padded cells of level tl
 };
 
 template <class T>
 __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sbudget, BlockViews<T>* v) {
     size_t goff = 0, soff = 0;
-    auto gtake = [&](size_t bytes) -> char* {
-        char* ptr = gbase ? gbase + goff : nullptr;
-        goff += (bytes + 255) & ~(size_t)255;
+    // `lead` and `trail` bytes of guard around an array of `bytes` (multiples of 16)
+    auto gtake = [&](size_t lead, size_t bytes, size_t trail) -> char* {
+        char* ptr = gbase ? gbase + goff + ((lead + 255) & ~(size_t)255) : nullptr;
+        goff += ((lead + 255) & ~(size_t)255) + ((bytes + trail + 255) & ~(size_t)255);
         return ptr;
     };
-    auto stake = [&](size_t bytes) -> char* {
-        char* ptr = sbase ? sbase + soff : nullptr;
-        soff += (bytes + 15) & ~(size_t)15;
-        return ptr;
+    auto take = [&](size_t lead, size_t bytes, size_t trail) -> char* {
+        lead = (lead + 15) & ~(size_t)15;
+        const size_t all = lead + ((bytes + trail + 15) & ~(size_t)15);
+        if (soff + all <= sbudget) {
+            char* ptr = sbase ? sbase + soff + lead : nullptr;
+            soff += all;
+            return ptr;
+        }
+        return gtake(lead, bytes, trail);
     };
-    int sides[kMaxLevels];
+    int sides[kBlockLevels];
     int nlev = 0;
-    for (int s = n; nlev < kMaxLevels;) {
+    for (int s = n; nlev < kBlockLevels;) {
         sides[nlev++] = s;
         if (s <= 1) break;
         s = (s + 1) / 2;
@@ -84,30 +94,11 @@ __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sb
             tl = l;
             break;
         }
-    const int ntail = tl ? sides[tl] * sides[tl] : 0;
-    const int cyc_levels = tl ? tl : nlev;  // levels the cycle itself visits
     const bool fp32 = sizeof(T) == 4;
-    // Shared memory, in order of the traffic it saves: level 0's cycle data
-    // when the whole of it fits (a visit of level l moves ~4^-l of level 0's
-    // bytes and happens 2^l times per W-cycle, so level 0 carries about half
-    // of a cycle's traffic: the coefficient copies, and for an FP32 cycle its
-    // iterate and right-hand side too); then the tail operator (with level
-    // tl's x and b, which it reads and writes); then the coarsest cycle levels
-    // that still fit.
-    auto arr = [](size_t cells) { return ((cells * sizeof(T) + 15) & ~(size_t)15); };
-    const size_t l0_bytes = (fp32 ? 6 : 4) * arr((size_t)n * n);
-    const bool l0_shared = nlev > 1 && cyc_levels >= 1 && l0_bytes <= sbudget;
-    size_t need = l0_shared ? l0_bytes : 0;
-    const size_t tail_bytes = tl ? arr((size_t)ntail * ntail) + 2 * arr((size_t)ntail) : 0;
-    const bool tail_shared = tl && need + tail_bytes <= sbudget;
-    if (tail_shared) need += tail_bytes;
-    int ls = cyc_levels;
-    for (int l = cyc_levels - 1; l >= 1; --l) {
-        const size_t lvl = 6 * (((size_t)sides[l] * sides[l] * sizeof(T) + 15) & ~(size_t)15);
-        if (need + lvl > sbudget) break;
-        need += lvl;
-        ls = l;
-    }
+    const size_t w = sizeof(T);
+    auto padded = [&](int l) { return (size_t)(2 * ((sides[l] + 1) / 2)); };
+    const int ntail = tl ? (int)(padded(tl) * padded(tl)) : 0;
+    const int cyc_levels = tl ? tl : nlev;  // levels the cycle itself visits
     if (v) {
         v->nlev = nlev;
         v->tl = tl;
@@ -115,72 +106,79 @@ __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sb
         v->tail = nullptr;
     }
     if (tl) {
-        T* tp = (T*)(tail_shared ? stake(sizeof(T) * (size_t)ntail * ntail)
-                                 : gtake(sizeof(T) * (size_t)ntail * ntail));
+        T* tp = (T*)take(0, w * (size_t)ntail * tail_pitch<T>(ntail), 0);
         if (v) v->tail = tp;
     }
-    const size_t m0 = (size_t)n * n;
     for (int l = 0; l < nlev; ++l) {
-        const size_t m = (size_t)sides[l] * sides[l];
+        const size_t np = padded(l), m = np * np;
         Lvl64 H;
         H.n = sides[l];
-        H.e = (double*)gtake(8 * m);
-        H.nf = (double*)gtake(8 * m);
-        H.d = (double*)gtake(8 * m);
-        H.id = (double*)gtake(8 * m);
-        H.wb = (double*)gtake(8 * (size_t)sides[l]);
-        H.sb = (double*)gtake(8 * (size_t)sides[l]);
+        H.e = (double*)gtake(16, 8 * m, 0);
+        H.nf = (double*)gtake(8 * np, 8 * m, 0);
+        H.d = (double*)gtake(0, 8 * m, 0);
+        H.id = (double*)gtake(0, 8 * m, 0);
+        H.wb = (double*)gtake(0, 8 * (size_t)sides[l], 0);
+        H.sb = (double*)gtake(0, 8 * (size_t)sides[l], 0);
         if (v) v->h[l] = H;
     }
-    double* cgv[5];
-    for (int q = 0; q < 5; ++q) cgv[q] = (double*)gtake(8 * m0);
-    if (v)
-        for (int q = 0; q < 5; ++q) v->cg[q] = cgv[q];
-    for (int l = 0; l < nlev; ++l) {
-        const size_t m = (size_t)sides[l] * sides[l];
-        Lvl<T> V{};
+    const size_t np0 = padded(0), m0 = np0 * np0;
+    {
+        double* p = (double*)gtake(8 * np0, 8 * m0, 8 * np0);
+        double* ap = (double*)gtake(0, 8 * m0, 0);
+        double* u = (double*)gtake(8 * np0, 8 * m0, 8 * np0);
+        double* r = fp32 ? (double*)gtake(0, 8 * m0, 0) : nullptr;
+        if (v) {
+            v->p = p;
+            v->ap = ap;
+            v->u = u;
+            v->r = r;
+        }
+    }
+    for (int l = nlev - 1; l >= 0; --l) {
+        const size_t np = padded(l), m = np * np;
+        PLvl<T> V{};
         V.n = sides[l];
-        if (tl && l > tl) {  // inside the tail: never visited by the cycle
-            if (v) v->lv[l] = V;
-            continue;
-        }
-        const bool shared = (l == 0 && l0_shared) || (l >= ls && l < cyc_levels) || (tail_shared && l == tl);
-        auto take = [&](size_t bytes) { return shared ? stake(bytes) : gtake(bytes); };
-        if (l < cyc_levels) {
-            if (fp32 || shared) {
-                V.e = (const T*)take(sizeof(T) * m);
-                V.nf = (const T*)take(sizeof(T) * m);
-                V.d = (const T*)take(sizeof(T) * m);
-                V.id = (const T*)take(sizeof(T) * m);
-            } else if (v) {
-                V.e = (const T*)v->h[l].e;
-                V.nf = (const T*)v->h[l].nf;
-                V.d = (const T*)v->h[l].d;
-                V.id = (const T*)v->h[l].id;
+        V.nc = (int)(np / 2);
+        V.np = (int)np;
+        V.rcp = row_reciprocal(V.nc);
+        if (!tl || l <= tl) {
+            // most read first: the iterate (every pass reads five values a
+            // cell), the faces, 1/d and the right-hand side, d (residual only)
+            V.x = (T*)take(w * np, w * m, w * np);
+            if (l < cyc_levels) {
+                // (FP64: the hierarchy itself where shared memory has no room)
+                auto coeff = [&](size_t lead, const double* h) -> const T* {
+                    const size_t ld = (lead + 15) & ~(size_t)15, all = ld + ((w * m + 15) & ~(size_t)15);
+                    if (!fp32 && soff + all > sbudget) return (const T*)h;
+                    return (const T*)take(lead, w * m, 0);
+                };
+                V.e = coeff(16, v ? v->h[l].e : nullptr);
+                V.nf = coeff(w * np, v ? v->h[l].nf : nullptr);
+                V.id = coeff(0, v ? v->h[l].id : nullptr);
+                V.b = (T*)take(0, w * m, 0);
+                V.d = coeff(0, v ? v->h[l].d : nullptr);
+            } else {
+                V.b = (T*)take(0, w * m, 0);  // the tail's input
             }
-        }
-        if (l == 0 && !fp32) {
-            V.x = (T*)cgv[4];  // z
-            V.b = (T*)cgv[1];  // r
-        } else {
-            // level tl (the tail's input/output) only needs x and b
-            V.x = (T*)take(sizeof(T) * m);
-            V.b = (T*)take(sizeof(T) * m);
         }
         if (v) v->lv[l] = V;
     }
+    if (v && !fp32) v->r = (double*)v->lv[0].b;
     if (tl) {  // tail construction scratch: every tail level with ntail right-hand sides
         for (int l = tl; l < nlev; ++l) {
-            const size_t m = (size_t)sides[l] * sides[l];
-            Lvl<T> M{};
+            const size_t np = padded(l), m = np * np, st = (size_t)rhs_stride((int)np);
+            PLvl<T> M{};
             M.n = sides[l];
-            M.x = (T*)gtake(sizeof(T) * m * ntail);
-            M.b = (T*)gtake(sizeof(T) * m * ntail);
+            M.nc = (int)(np / 2);
+            M.np = (int)np;
+            M.rcp = row_reciprocal(M.nc);
+            M.x = (T*)gtake(w * np, w * st * ntail, 0);
+            M.b = (T*)gtake(w * np, w * st * ntail, 0);
             if (fp32) {
-                M.e = (const T*)gtake(sizeof(T) * m);
-                M.nf = (const T*)gtake(sizeof(T) * m);
-                M.d = (const T*)gtake(sizeof(T) * m);
-                M.id = (const T*)gtake(sizeof(T) * m);
+                M.e = (const T*)gtake(16, w * m, 0);
+                M.nf = (const T*)gtake(w * np, w * m, 0);
+                M.d = (const T*)gtake(0, w * m, 0);
+                M.id = (const T*)gtake(0, w * m, 0);
             } else if (v) {
                 M.e = (const T*)v->h[l].e;
                 M.nf = (const T*)v->h[l].nf;
@@ -190,134 +188,248 @@ __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sb
             if (v) v->lm[l] = M;
         }
     }
-    return BlockLayout{goff, soff, nlev, ls};
+    return BlockLayout{goff, soff, nlev};
+}
+
+// Zeroes what the stencils may read before a pass has written it: the guards
+// around the arrays, the iterates (at the end of a row a pass reads the next
+// row's first cell, times a zero face, which must be finite), the padding of
+// r, u and the coarse right-hand sides. Needed once per layout (no pass writes
+// a guard, padding stays zero) and after a problem that left non-finite values.
+template <class T>
+__device__ void block_clear(const BlockViews<T>& V) {
+    const int t0 = threadIdx.x, ts = blockDim.x;
+    auto zero = [&](auto* ptr, int count) {
+        for (int t = t0; t < count; t += ts) ptr[t] = 0;
+    };
+    for (int l = 0; l < V.nlev; ++l) {
+        const Lvl64& H = V.h[l];
+        const int np = 2 * ((H.n + 1) / 2), m = np * np;
+        zero(H.e - 2, 2);
+        zero(H.nf - np, np);
+        const PLvl<T>& A = V.lv[l];
+        if (A.x) {
+            zero(A.x - np, m + 2 * np);
+            zero(A.b, m);
+        }
+        if (A.e) {
+            zero((T*)A.e - 2, 2);
+            zero((T*)A.nf - np, np);
+        }
+        if (V.tl && l >= V.tl) {
+            const PLvl<T>& M = V.lm[l];
+            zero(M.x - np, rhs_stride(np) * V.ntail);
+            zero(M.b - np, rhs_stride(np) * V.ntail);
+            zero((T*)M.e - 2, 2);
+            zero((T*)M.nf - np, np);
+        }
+    }
+    const int np = V.lv[0].np, m = np * np;
+    zero(V.p - np, np);
+    zero(V.p + m, np);
+    zero(V.u - np, m + 2 * np);
+    zero(V.r, m);
+    __syncthreads();
+}
+
+// The fine level (level.hpp:79-97, validation solver.hpp:68-77) with every
+// face computed once (one division per face instead of two; FP64 division is
+// tens of instructions on the narrow FP64 pipe): the east/north faces and the
+// boundary faces first, then the diagonal from the stored faces in
+// build_fine's summation order. A cell's west/south face is its neighbour's
+// east/north face, the same bits since harmonic() is symmetric, so the level
+// equals build_fine's bit for bit. with_id false leaves id unwritten (the
+// FP32 cycle computes its own reciprocal from the FP32 diagonal). `a` has
+// pitch n, the level the padded pitch.
+__device__ __forceinline__ void block_build_fine(const double* __restrict__ a, const Lvl64& L,
+                                                 unsigned long long* bad, bool with_id) {
+    const int n = L.n, np = 2 * ((n + 1) / 2), m = np * np;
+    for (int c = threadIdx.x; c < m; c += blockDim.x) {
+        const int i = c / np, j = c - i * np;
+        double e = 0.0, nf = 0.0;
+        if (i < n && j < n) {
+            const int64_t k = (int64_t)i * n + j;
+            const double ac = a[k];
+            if (!(ac > 0.0) || !isfinite(ac)) atomicMin(bad, (unsigned long long)k);
+            e = (j + 1 < n) ? harmonic(ac, a[k + 1]) : ac;
+            nf = (i + 1 < n) ? harmonic(ac, a[k + n]) : ac;
+            if (j == 0) L.wb[i] = ac;
+            if (i == 0) L.sb[j] = ac;
+        }
+        L.e[c] = e;
+        L.nf[c] = nf;
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < m; c += blockDim.x) {
+        const int i = c / np, j = c - i * np;
+        double dd = 0.0, id = 0.0;
+        if (i < n && j < n) {
+            const double w = (j > 0) ? L.e[c - 1] : L.wb[i];
+            const double s = (i > 0) ? L.nf[c - np] : L.sb[j];
+            dd = L.e[c] + w + L.nf[c] + s;
+            if (with_id) id = 1.0 / dd;
+        }
+        L.d[c] = dd;
+        if (with_id) L.id[c] = id;
+    }
+    __syncthreads();
+}
+
+// Galerkin coarse operator (coarsen in setup.cuh) between padded levels.
+__device__ __forceinline__ void block_coarsen(const Lvl64& F, const Lvl64& C, bool with_id) {
+    const int n = F.n, np = 2 * ((n + 1) / 2), nc = C.n, npc = 2 * ((nc + 1) / 2), mc = npc * npc;
+    for (int c = threadIdx.x; c < mc; c += blockDim.x) {
+        const int I = c / npc, J = c - I * npc;
+        double ce = 0.0, cw = 0.0, cn = 0.0, cs = 0.0, dd = 0.0, id = 0.0;
+        if (I < nc && J < nc) {
+            const int i0 = 2 * I, i1 = (2 * I + 1 < n) ? 2 * I + 1 : 2 * I;
+            const int j0 = 2 * J, j1 = (2 * J + 1 < n) ? 2 * J + 1 : 2 * J;
+            for (int i = i0; i <= i1; ++i) {
+                ce += F.e[i * np + j1];
+                cw += (j0 > 0) ? F.e[i * np + j0 - 1] : F.wb[i];
+            }
+            for (int j = j0; j <= j1; ++j) {
+                cn += F.nf[i1 * np + j];
+                cs += (i0 > 0) ? F.nf[(i0 - 1) * np + j] : F.sb[j];
+            }
+            dd = ce + cw + cn + cs;
+            if (with_id) id = 1.0 / dd;
+            if (J == 0) C.wb[I] = cw;
+            if (I == 0) C.sb[J] = cs;
+        }
+        C.e[c] = ce;
+        C.nf[c] = cn;
+        C.d[c] = dd;
+        if (with_id) C.id[c] = id;
+    }
+}
+
+// The faces on the domain's east and north boundary enter d and the coarser
+// levels' faces only; zero, they drop out of every stencil (patch.cuh).
+__device__ __forceinline__ void block_drop_boundary(const Lvl64& L) {
+    const int n = L.n, np = 2 * ((n + 1) / 2);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        L.e[t * np + n - 1] = 0.0;
+        L.nf[(n - 1) * np + t] = 0.0;
+    }
 }
 
 // Cycle coefficients of level l in the cycle's precision (FP32 copies for the
-// mixed form, shared-memory copies for the levels held on chip). The FP32
+// mixed form, shared-memory copies for FP64 arrays held on chip). The FP32
 // reciprocal diagonal is the correctly rounded reciprocal of the FP32 d (the
 // FP64 id, one FP64 division per cell, is built for FP32 cycles on the
 // coarsest level only); FP64 copies take id as built.
 template <class T>
-__device__ __forceinline__ void block_copy_coeffs(const Lvl64& H, const Lvl<T>& V) {
-    if (!V.e || (const void*)V.e == (const void*)H.e) return;  // not visited / FP64 used in place
-    const int64_t m = (int64_t)H.n * H.n;
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-        ((T*)V.e)[k] = narrow_to<T>(H.e[k]);
-        ((T*)V.nf)[k] = narrow_to<T>(H.nf[k]);
-        const T dk = narrow_to<T>(H.d[k]);
-        ((T*)V.d)[k] = dk;
-        if constexpr (sizeof(T) == 4)
-            ((T*)V.id)[k] = __frcp_rn(dk);
-        else
-            ((T*)V.id)[k] = H.id[k];
+__device__ __forceinline__ void block_copy_coeffs(const Lvl64& H, const PLvl<T>& V) {
+    if (!V.e) return;  // not visited
+    const int m = V.np * V.np;
+    if constexpr (sizeof(T) == 4) {
+        for (int k = threadIdx.x; k < m; k += blockDim.x) {
+            ((T*)V.e)[k] = narrow_to<T>(H.e[k]);
+            ((T*)V.nf)[k] = narrow_to<T>(H.nf[k]);
+            const T dk = narrow_to<T>(H.d[k]);
+            ((T*)V.d)[k] = dk;
+            // (FP64 zero, tested off the FP64 pipe: a cell outside the domain)
+            ((T*)V.id)[k] = __double_as_longlong(H.d[k]) != 0 ? __frcp_rn(dk) : T(0);
+        }
+    } else {
+        auto copy = [&](const T* to, const double* from) {
+            if ((const double*)to == from) return;
+            for (int k = threadIdx.x; k < m; k += blockDim.x) ((T*)to)[k] = from[k];
+        };
+        copy(V.e, H.e);
+        copy(V.nf, H.nf);
+        copy(V.d, H.d);
+        copy(V.id, H.id);
     }
+}
+
+// y = A x of two horizontally adjacent cells (pair q of a padded level of
+// pitch 2 * n2), terms in apply_cell's order.
+__device__ __forceinline__ double2 pair_apply(const Lvl64& L, const double* __restrict__ x, int q, int n2,
+                                              double2 xc) {
+    const double2* x2 = reinterpret_cast<const double2*>(x);
+    const double2* nf2 = reinterpret_cast<const double2*>(L.nf);
+    const double2 dd = reinterpret_cast<const double2*>(L.d)[q], ee = reinterpret_cast<const double2*>(L.e)[q];
+    const double2 nn = nf2[q], ns = nf2[q - n2], xn = x2[q + n2], xs = x2[q - n2];
+    double v0 = dd.x * xc.x, v1 = dd.y * xc.y;
+    v0 -= ee.x * xc.y;
+    v1 -= ee.y * x[2 * q + 2];
+    v0 -= L.e[2 * q - 1] * x[2 * q - 1];
+    v1 -= ee.x * xc.x;
+    v0 -= nn.x * xn.x;
+    v1 -= nn.y * xn.y;
+    v0 -= ns.x * xs.x;
+    v1 -= ns.y * xs.y;
+    return make_double2(v0, v1);
 }
 
 // y = A x over a block, FP64, returning sum x . y.
 __device__ __forceinline__ double block_apply_dot(const Lvl64& L, const double* x, double* y, double* red) {
-    const int n = L.n;
-    const int64_t m = (int64_t)n * n;
+    const int n2 = (L.n + 1) / 2, m2 = 2 * n2 * n2;
     double acc = 0.0;
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-        const int i = (int)k / n, j = (int)k - i * n;  // n^2 < 2^31
-        const double v = apply_cell(L, x, i, j);
-        y[k] = v;
-        acc += x[k] * v;
+    for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+        const double2 xc = reinterpret_cast<const double2*>(x)[q];
+        const double2 v = pair_apply(L, x, q, n2, xc);
+        reinterpret_cast<double2*>(y)[q] = v;
+        acc += xc.x * v.x;
+        acc += xc.y * v.y;
     }
     return block_sum_wide(acc, red);
 }
 
-// The same for an even side, two horizontally adjacent cells per thread with
-// 16-byte loads and stores (twice the bytes in flight per load instruction for
-// this latency-bound loop); each cell's terms in apply_cell's order. All
-// arrays 16-byte aligned (the arena's).
-__device__ __forceinline__ double block_apply_dot2(const Lvl64& L, const double* x, double* y, double* red) {
-    const int n = L.n, n2 = n >> 1;
-    const int64_t m2 = (int64_t)n * n2;
-    const double2* x2 = reinterpret_cast<const double2*>(x);
-    const double2* d2 = reinterpret_cast<const double2*>(L.d);
-    const double2* e2 = reinterpret_cast<const double2*>(L.e);
-    const double2* nf2 = reinterpret_cast<const double2*>(L.nf);
-    double acc = 0.0;
-    for (int64_t q = threadIdx.x; q < m2; q += blockDim.x) {
-        const int i = (int)q / n2, jp = (int)q - i * n2, j = 2 * jp;  // n^2 < 2^31
-        const int64_t k = (int64_t)i * n + j;
-        const double2 xc = x2[q], dd = d2[q], ee = e2[q];
-        double v0 = dd.x * xc.x, v1 = dd.y * xc.y;
-        v0 -= ee.x * xc.y;                            // east of j (j + 1 < n: j even, n even)
-        if (j > 0) v0 -= L.e[k - 1] * x[k - 1];       // west of j
-        if (j + 2 < n) v1 -= ee.y * x[k + 2];         // east of j + 1
-        v1 -= ee.x * xc.x;                            // west of j + 1
-        if (i + 1 < n) {
-            const double2 nn = nf2[q], xn = x2[q + n2];
-            v0 -= nn.x * xn.x;
-            v1 -= nn.y * xn.y;
-        }
-        if (i > 0) {
-            const double2 ns = nf2[q - n2], xs = x2[q - n2];
-            v0 -= ns.x * xs.x;
-            v1 -= ns.y * xs.y;
-        }
-        reinterpret_cast<double2*>(y)[q] = make_double2(v0, v1);
-        acc += xc.x * v0;
-        acc += xc.y * v1;
-    }
-    return block_sum_wide(acc, red);
-}
-
-// z = M r for one problem; returns r . z. For the FP32 cycle, r is rounded
-// into the level-0 right-hand side and the FP32 iterate widened into z.
+// b = r in the cycle's precision and the cycle's first pass (colour 0 from a
+// zero iterate) for pair q. The two cells of a pair are one of each colour.
 template <class T>
-__device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V, const double* r, double* z,
-                                     double* red, bool b_ready = false) {
-    const int n = V.h[0].n;
-    const int64_t m = (int64_t)n * n;
+__device__ __forceinline__ void pair_start_cycle(const PLvl<T>& L, int q, double2 rv) {
+    const int odd = patch_row(q, L.nc, L.rcp) & 1;  // n2 = nc pairs a row: the row's parity
+    const T b0 = narrow_to<T>(rv.x), b1 = narrow_to<T>(rv.y);
+    if constexpr (sizeof(T) == 4) {  // (FP64: b is r itself)
+        Pair_t<T> bb;
+        bb.x = b0;
+        bb.y = b1;
+        reinterpret_cast<Pair_t<T>*>(L.b)[q] = bb;
+    }
+    L.x[2 * q + odd] = (odd ? b1 : b0) * L.id[2 * q + odd];
+}
+
+// z = M r for one problem, r already handed over by pair_start_cycle on every
+// pair (multigrid) and the CTA synchronised since; returns r . z. The
+// cycle's iterate lv[0].x is z, in the cycle's precision.
+template <class T>
+__device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V, double* red) {
+    const PLvl<T>& L = V.lv[0];
+    const double* r = V.r;
     double acc = 0.0;
     if (A.pc == kPcMultigrid) {
-        const double* id64 = V.h[V.nlev - 1].id;  // FP64 exact coarsest solve (no-tail hierarchies)
-        if (sizeof(T) == 4) {
-            if (!b_ready) {  // (the CG update usually wrote the rounded r already)
-                for (int64_t k = threadIdx.x; k < m; k += blockDim.x) V.lv[0].b[k] = narrow_to<T>(r[k]);
-                __syncthreads();
-            }
-            block_cycle<T>(V.lv, 0, V.nlev, A.pre, A.post, A.gamma, 1, id64, V.tail, V.tl);
-            if ((m & 1) == 0) {  // pairs: 8-byte FP32 and 16-byte FP64 accesses (arena-aligned)
-                const float2* x2 = reinterpret_cast<const float2*>(V.lv[0].x);
-                const double2* r2 = reinterpret_cast<const double2*>(r);
-                for (int64_t q = threadIdx.x; q < (m >> 1); q += blockDim.x) {
-                    const float2 xx = x2[q];
-                    const double2 rr = r2[q];
-                    const double z0 = widen_f32(xx.x), z1 = widen_f32(xx.y);
-                    reinterpret_cast<double2*>(z)[q] = make_double2(z0, z1);
-                    acc += rr.x * z0;
-                    acc += rr.y * z1;
-                }
-            } else {
-                for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-                    const double zk = widen_f32(V.lv[0].x[k]);
-                    z[k] = zk;
-                    acc += r[k] * zk;
-                }
+        const double* id64 = sizeof(T) == 4 ? V.h[V.nlev - 1].id : nullptr;  // FP64 exact coarsest solve
+        if (V.nlev == 1) {  // one cell, solved exactly
+            if (threadIdx.x == 0) {
+                L.x[0] = id64 ? (T)((double)L.b[0] * id64[0]) : L.b[0] * L.id[0];
+                acc = r[0] * widen_f32(L.x[0]);
             }
         } else {
-            block_cycle<T>(V.lv, 0, V.nlev, A.pre, A.post, A.gamma, 1, nullptr, V.tail, V.tl);
-            if ((m & 1) == 0) {
-                const double2* r2 = reinterpret_cast<const double2*>(r);
-                const double2* z2 = reinterpret_cast<const double2*>(z);
-                for (int64_t q = threadIdx.x; q < (m >> 1); q += blockDim.x) {
-                    const double2 rr = r2[q], zz = z2[q];
-                    acc += rr.x * zz.x;
-                    acc += rr.y * zz.y;
-                }
-            } else {
-                for (int64_t k = threadIdx.x; k < m; k += blockDim.x) acc += r[k] * z[k];
+            patch_cycle<T>(V.lv, V.nlev, A.pre, A.post, A.gamma, id64, V.tail, V.tl);
+            // the last colour-0 pass and r . z
+            const int nc = L.nc, cnt = nc * nc, np = L.np;
+            for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+                const int k = 2 * q + 2 * patch_row(q, nc, L.rcp) * nc;
+                T o0, o1;
+                patch_red(L, L.x, L.b, k, o0, o1);
+                L.x[k] = o0;
+                L.x[k + np + 1] = o1;
+                const double2 r0 = load_pair(r + k), r1 = load_pair(r + k + np);
+                acc += r0.x * widen_f32(o0);
+                acc += r0.y * widen_f32(L.x[k + 1]);
+                acc += r1.x * widen_f32(L.x[k + np]);
+                acc += r1.y * widen_f32(o1);
             }
         }
-    } else {
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
+    } else {  // (FP64 only)
+        const int m = L.np * L.np;
+        for (int k = threadIdx.x; k < m; k += blockDim.x) {
             const double zk = A.pc == kPcJacobi ? r[k] * V.h[0].id[k] : r[k];
-            z[k] = zk;
+            L.x[k] = (T)zk;
             acc += r[k] * zk;
         }
     }
@@ -326,21 +438,23 @@ __device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V,
 
 // The dense tail of one problem: column j = the tail map applied to e_j, all
 // columns at once, in the cycle's precision (the FP32 smoothing of the mixed
-// form, with the exact 1 x 1 coarsest solve in FP64), stored row-major.
+// form, with the exact 1 x 1 coarsest solve in FP64), stored row-major; rows
+// and columns of padding cells are zero.
 // Building it in FP64 cost the mixed form about a third of its FP64 work.
 template <class T>
 __device__ void block_build_tail(const BatchArgs& A, const BlockViews<T>& V) {
-    const int tl = V.tl, N = V.ntail;
-    const Lvl<T>& L = V.lm[tl];
+    const int tl = V.tl, N = V.ntail, pitch = tail_pitch<T>(N);
+    const PLvl<T>& L = V.lm[tl];
+    const int st = rhs_stride(L.np);
     for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
         const int j = t / N, k = t - j * N;  // right-hand side j, cell k
-        L.b[t] = (k == j) ? T(1) : T(0);
+        L.b[j * st + k] = (k == j && j / L.np < L.n && j % L.np < L.n) ? T(1) : T(0);
     }
     __syncthreads();
-    block_cycle_m<T>(V.lm, tl, V.nlev, A.pre, A.post, A.gamma, A.gamma, N, V.h[V.nlev - 1].id);
+    patch_cycle_m<T>(V.lm, tl, V.nlev, A.pre, A.post, A.gamma, N, sizeof(T) == 4 ? V.h[V.nlev - 1].id : nullptr);
     for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
         const int j = t / N, k = t - j * N;
-        V.tail[k * N + j] = L.x[t];
+        V.tail[k * pitch + j] = L.x[j * st + k];
     }
     __syncthreads();
 }
@@ -355,11 +469,14 @@ __device__ unsigned long long block_setup(const BatchArgs& A, const double* a, c
     // FP64 reciprocal diagonals: every level for an FP64 cycle; level 0 for
     // the Jacobi preconditioner; otherwise the coarsest level's exact solve only.
     const bool fp64_id = sizeof(T) == 8 || A.pc != kPcMultigrid;
-    build_fine_block(a, V.h[0], s_bad, fp64_id || V.nlev == 1);
+    block_build_fine(a, V.h[0], s_bad, fp64_id || V.nlev == 1);
     for (int l = 1; l < V.nlev; ++l) {
-        coarsen<BlockScope>(V.h[l - 1], V.h[l], fp64_id || l == V.nlev - 1);
+        block_coarsen(V.h[l - 1], V.h[l], fp64_id || l == V.nlev - 1);
         __syncthreads();
+        block_drop_boundary(V.h[l - 1]);  // (read by the coarsening just done)
     }
+    block_drop_boundary(V.h[V.nlev - 1]);
+    __syncthreads();
     if (A.pc == kPcMultigrid) {
         for (int l = 0; l < V.nlev; ++l) block_copy_coeffs<T>(V.h[l], V.lv[l]);
         for (int l = V.tl ? V.tl : V.nlev; l < V.nlev; ++l) block_copy_coeffs<T>(V.h[l], V.lm[l]);

@@ -920,7 +920,11 @@ void launch_copy_back(const T* src, double* dst, int64_t m, cudaStream_t s) {
 
 // ================================================================ block engine
 
-int num_levels_for(int n) { return carve<double>(n, nullptr, nullptr, 0, nullptr).nlev; }
+int num_levels_for(int n) {
+    int l = 1;
+    for (; n > 1 && l < kMaxLevels; ++l) n = (n + 1) / 2;
+    return l;
+}
 
 size_t block_arena_bytes(int n, bool mixed, size_t sbudget) {
     return mixed ? carve<float>(n, nullptr, nullptr, sbudget, nullptr).global_bytes
@@ -928,16 +932,28 @@ size_t block_arena_bytes(int n, bool mixed, size_t sbudget) {
 }
 
 // One whole PCG solve (solver.hpp:83-174) by one CTA.
+//
+// The loops over cells that need no neighbour walk pairs of horizontally
+// adjacent cells of the padded level; the same thread owns the same pairs in
+// all of them. Level 0's first smoothing pass rides on the loop that updates
+// r, its last one on the r . z product (block_precondition), so an iteration
+// reads r, b and the iterate twice less often and has two barriers fewer.
+// Bound by the latency of its barrier-separated passes (FP32 cycle) and the
+// FP64 pipe. On GB300, against the cell-by-cell passes it replaces (256
+// threads, 48 KiB; device time): 4096 x 64^2 mixed 19.6 -> 14.7 ms, FP64 41 ->
+// 31.7 ms, 512 x 128^2 at contrast 1e4 FP64 36 -> 31 ms (512 threads).
+// Returns false when the solve broke down (the arena may hold non-finite
+// values).
 template <class T>
-__device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>& V, double* red,
+__device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>& V, double* red,
                                 unsigned long long* s_bad) {
     const int n = A.side[pid];
-    const int64_t m = (int64_t)n * n;
     const int64_t off = A.off[pid];
-    double* u = A.u + off;
-    double *b = V.cg[0], *r = V.cg[1], *p = V.cg[2], *ap = V.cg[3], *z = V.cg[4];
-    const Lvl64* h = V.h;
-    const int nlev = V.nlev;
+    double *r = V.r, *p = V.p, *ap = V.ap, *u = V.u;
+    const Lvl64& h0 = V.h[0];
+    const PLvl<T>& L0 = V.lv[0];
+    const int np = L0.np, m2 = np * (np / 2);
+    const bool mg = A.pc == kPcMultigrid;
 
     const unsigned long long bad = block_setup<T>(A, A.a + off, V, s_bad);
     if (bad != ~0ull) {
@@ -949,7 +965,7 @@ __device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             A.levels[pid] = 1;
             if (A.true_residual) A.true_residual[pid] = 0.0;
         }
-        return;
+        return false;
     }
 
     const double hh = 1.0 / (double)(n + 1);
@@ -957,24 +973,23 @@ __device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     const double* f = A.f ? (A.f_shared ? A.f : A.f + off) : nullptr;
     const double* u0 = A.u0 ? A.u0 + off : nullptr;
     const bool record = A.record_history && A.history && A.count == 1;
-    // Standard beta, as in the grid engine (the flexible variant measured
-    // worse for the FP32 cycle).
-    constexpr bool flexible = false;
+    auto rhs = [&](int k) { return (f ? f[k] : A.fscalar) * h2; };  // cell k of the packed arrays
+    double* u_out = A.u + off;
 
     double sb = 0.0;
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-        const double bk = (f ? f[k] : A.fscalar) * h2;
-        b[k] = bk;
-        u[k] = u0 ? u0[k] : 0.0;
+    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
+        const int i = k / n, c = i * np + (k - i * n);
+        const double bk = rhs(k);
+        r[c] = bk;
+        u[c] = u0 ? u0[k] : 0.0;
         sb += bk * bk;
     }
     const double bnorm = sqrt(block_sum_wide(sb, red));
     int iterations = 0, converged = 0;
+    bool sound = true;
     double residual = 0.0;
     if (bnorm == 0.0) {
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-            u[k] = 0.0;
-        }
+        for (int k = threadIdx.x; k < n * n; k += blockDim.x) u_out[k] = 0.0;
         if (threadIdx.x == 0) {
             A.bad[pid] = ~0ull;
             A.iterations[pid] = 0;
@@ -983,35 +998,39 @@ __device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             A.levels[pid] = 1;
             if (A.true_residual) A.true_residual[pid] = 0.0;
         }
-        return;
+        return true;
     }
 
     double bu0 = 0.0;  // b . u0: estimates the solution's energy ||u||_A^2 = b . u for a close u0
+    residual = 1.0;
     if (u0) {
         double sr = 0.0, sbu = 0.0;
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-            const int i = (int)k / n, j = (int)k - i * n;  // n^2 < 2^31
-            const double rk = b[k] - apply_cell(h[0], u, i, j);
-            r[k] = rk;
-            sr += rk * rk;
-            sbu += b[k] * u[k];
+        for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+            const double2 uu = load_pair(u + 2 * q), bb = load_pair(r + 2 * q);
+            const double2 au = pair_apply(h0, u, q, np / 2, uu);
+            const double2 rv = make_double2(bb.x - au.x, bb.y - au.y);
+            reinterpret_cast<double2*>(r)[q] = rv;
+            sr += rv.x * rv.x;
+            sr += rv.y * rv.y;
+            sbu += bb.x * uu.x;
+            sbu += bb.y * uu.y;
         }
         residual = sqrt(block_sum_wide(sr, red)) / bnorm;
         if (A.u0_fallback) bu0 = block_sum_wide(sbu, red);
-    } else {
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) r[k] = b[k];
-        residual = 1.0;
-        __syncthreads();
     }
     if (record && threadIdx.x == 0) A.history[0] = residual;
 
+    auto start_cycle = [&] {  // r in place: b and the cycle's first pass
+        if (mg)
+            for (int q = threadIdx.x; q < m2; q += blockDim.x) pair_start_cycle<T>(L0, q, load_pair(r + 2 * q));
+        __syncthreads();
+    };
     if (residual < A.tol) {
         converged = 1;
     } else {
-        // (Leaving z in the FP32 iterate and widening it where p reads it, with
-        // no FP64 z array, measured 2% slower: 4096 x 64^2 mixed 23.1 against
-        // 22.7 ms.)
-        double rz = block_precondition<T>(A, V, r, z, red);
+        __syncthreads();
+        start_cycle();
+        double rz = block_precondition<T>(A, V, red);
         // A predicted start no better than zero is dropped for the zero start,
         // the fallback it is judged against. CG minimises the error's energy
         // norm; r0 . M r0 (the first preconditioned residual, computed here
@@ -1019,89 +1038,62 @@ __device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         // solution's ||u||_A^2, so a start is kept while the first is below
         // the second. A rejected start costs one more cycle (z = M b).
         if (u0 && A.u0_fallback && !(rz < bu0)) {
-            for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-                u[k] = 0.0;
-                r[k] = b[k];
+            for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
+                const int i = k / n, c = i * np + (k - i * n);
+                u[c] = 0.0;
+                r[c] = rhs(k);
             }
             residual = 1.0;
             __syncthreads();
-            rz = block_precondition<T>(A, V, r, z, red);
+            start_cycle();
+            rz = block_precondition<T>(A, V, red);
         }
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) p[k] = z[k];
-        __syncthreads();
-        // Even sides take the paired loops: two cells per thread, 16-byte
-        // FP64 accesses (arena vectors are 256-byte aligned; u also needs an
-        // even offset in the packed output).
-        const bool pairs = (n & 1) == 0;
-        const bool pairs_u = pairs && (((uintptr_t)u) & 15) == 0;
+        double beta = 0.0;
         for (int it = 0; it < A.max_iter; ++it) {
-            const double pap = pairs ? block_apply_dot2(h[0], p, ap, red) : block_apply_dot(h[0], p, ap, red);
+            // p = z + beta p (z alone before the first iteration)
+            for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+                const Pair_t<T> zz = load_pair(L0.x + 2 * q);
+                double2 pp = make_double2(widen_f32(zz.x), widen_f32(zz.y));
+                if (it > 0) {
+                    const double2 old = load_pair(p + 2 * q);
+                    pp.x += beta * old.x;
+                    pp.y += beta * old.y;
+                }
+                reinterpret_cast<double2*>(p)[q] = pp;
+            }
+            __syncthreads();
+            const double pap = block_apply_dot(h0, p, ap, red);
             if (!(fabs(pap) > 0.0) || !isfinite(pap)) {
                 iterations = it;
                 converged = 0;
+                sound = false;
                 break;
             }
             const double alpha = rz / pap;
-            double rr = 0.0, rzo = 0.0;
-            // the FP32 cycle's input (r rounded) is written here, in the same pass
-            const bool round_b = sizeof(T) == 4 && A.pc == kPcMultigrid;
-            T* b32 = V.lv[0].b;
-            if (pairs_u && !flexible) {
-                double2* u2 = reinterpret_cast<double2*>(u);
-                double2* r2 = reinterpret_cast<double2*>(r);
-                const double2* p2 = reinterpret_cast<const double2*>(p);
-                const double2* a2 = reinterpret_cast<const double2*>(ap);
-                for (int64_t q = threadIdx.x; q < (m >> 1); q += blockDim.x) {
-                    double2 uu = u2[q], rv = r2[q];
-                    const double2 pp = p2[q], av = a2[q];
-                    uu.x += alpha * pp.x;
-                    uu.y += alpha * pp.y;
-                    rv.x = rv.x - alpha * av.x;
-                    rv.y = rv.y - alpha * av.y;
-                    u2[q] = uu;
-                    r2[q] = rv;
-                    rr += rv.x * rv.x;
-                    rr += rv.y * rv.y;
-                    if (round_b) {
-                        b32[2 * q] = narrow_to<T>(rv.x);
-                        b32[2 * q + 1] = narrow_to<T>(rv.y);
-                    }
-                }
-            } else {
-                for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-                    u[k] += alpha * p[k];
-                    const double rk = r[k] - alpha * ap[k];
-                    r[k] = rk;
-                    rr += rk * rk;
-                    if (round_b) b32[k] = narrow_to<T>(rk);
-                    if (flexible) rzo += rk * z[k];  // z still holds the previous direction's z
-                }
+            double rr = 0.0;
+            for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+                double2 uu = load_pair(u + 2 * q), rv = load_pair(r + 2 * q);
+                const double2 pp = load_pair(p + 2 * q), av = load_pair(ap + 2 * q);
+                uu.x += alpha * pp.x;
+                uu.y += alpha * pp.y;
+                rv.x = rv.x - alpha * av.x;
+                rv.y = rv.y - alpha * av.y;
+                reinterpret_cast<double2*>(u)[q] = uu;
+                reinterpret_cast<double2*>(r)[q] = rv;
+                rr += rv.x * rv.x;
+                rr += rv.y * rv.y;
+                if (mg) pair_start_cycle<T>(L0, q, rv);
             }
             residual = sqrt(block_sum_wide(rr, red)) / bnorm;
-            if (flexible) rzo = block_sum_wide(rzo, red);
             iterations = it + 1;
             if (record && threadIdx.x == 0) A.history[it + 1] = residual;
             if (residual < A.tol) {
                 converged = 1;
                 break;
             }
-            const double rz_new = block_precondition<T>(A, V, r, z, red, round_b);
-            const double beta = (rz_new - rzo) / rz;
+            const double rz_new = block_precondition<T>(A, V, red);
+            beta = rz_new / rz;
             rz = rz_new;
-            if (pairs) {
-                double2* p2 = reinterpret_cast<double2*>(p);
-                const double2* z2 = reinterpret_cast<const double2*>(z);
-                for (int64_t q = threadIdx.x; q < (m >> 1); q += blockDim.x) {
-                    const double2 zz = z2[q];
-                    double2 pp = p2[q];
-                    pp.x = zz.x + beta * pp.x;
-                    pp.y = zz.y + beta * pp.y;
-                    p2[q] = pp;
-                }
-            } else {
-                for (int64_t k = threadIdx.x; k < m; k += blockDim.x) p[k] = z[k] + beta * p[k];
-            }
-            __syncthreads();
         }
     }
 
@@ -1111,21 +1103,33 @@ __device__ void block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     __syncthreads();
     if (A.true_residual) {
         double tr = 0.0;
-        for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-            const int i = (int)k / n, j = (int)k - i * n;  // n^2 < 2^31
-            const double rk = b[k] - apply_cell(h[0], u, i, j);
-            tr += rk * rk;
+        for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+            const int i = 2 * q / np, j = 2 * q - i * np;
+            const double2 au = pair_apply(h0, u, q, np / 2, load_pair(u + 2 * q));
+            if (i < n) {
+                const double r0 = rhs(i * n + j) - au.x;
+                tr += r0 * r0;
+                if (j + 1 < n) {
+                    const double r1 = rhs(i * n + j + 1) - au.y;
+                    tr += r1 * r1;
+                }
+            }
         }
         true_res = sqrt(block_sum_wide(tr, red)) / bnorm;
+    }
+    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
+        const int i = k / n;
+        u_out[k] = u[i * np + (k - i * n)];
     }
     if (threadIdx.x == 0) {
         A.bad[pid] = ~0ull;
         A.iterations[pid] = iterations;
         A.converged[pid] = converged;
         A.residual[pid] = residual;
-        A.levels[pid] = A.pc == kPcMultigrid ? nlev : 1;
+        A.levels[pid] = mg ? V.nlev : 1;
         if (A.true_residual) A.true_residual[pid] = true_res;
     }
+    return sound && isfinite(residual);
 }
 
 // Dynamic shared memory of a block-engine CTA: the coarse-level budget, then
@@ -1143,16 +1147,22 @@ __global__ void __launch_bounds__(1024) k_block_solve(BatchArgs A) {
     extern __shared__ __align__(16) unsigned char block_smem[];
     double* red = reinterpret_cast<double*>(block_smem + block_red_offset(A.smem_budget));
     char* arena = A.scratch + (size_t)blockIdx.x * A.scratch_stride;
+    int carved = 0;  // the side the arena is laid out for
     for (;;) {
         if (threadIdx.x == 0) {
             const unsigned w = atomicAdd(A.work, 1u);
             s_pid = w < (unsigned)A.count ? A.order[w] : -1;
-            if (s_pid >= 0) carve<T>(A.side[s_pid], arena, (char*)block_smem, A.smem_budget, &V);
+            if (s_pid >= 0 && A.side[s_pid] != carved)
+                carve<T>(A.side[s_pid], arena, (char*)block_smem, A.smem_budget, &V);
         }
         __syncthreads();
         const int pid = s_pid;
         if (pid < 0) return;
-        block_solve_one<T>(A, pid, V, red, &s_bad);
+        if (A.side[pid] != carved) {
+            carved = A.side[pid];
+            block_clear<T>(V);
+        }
+        if (!block_solve_one<T>(A, pid, V, red, &s_bad)) carved = 0;
         __syncthreads();
     }
 }

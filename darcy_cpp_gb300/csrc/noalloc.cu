@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(256) k_precondition_noalloc(unsigned char* scr
     __shared__ unsigned long long s_bad;
     if (threadIdx.x == 0) carve<double>(n, (char*)scratch, nullptr, 0, &V);
     __syncthreads();
+    block_clear<double>(V);
     BatchArgs A{};
     A.pc = kPcMultigrid;
     A.pre = pre;
@@ -56,12 +57,14 @@ __global__ void __launch_bounds__(256) k_precondition_noalloc(unsigned char* scr
     unsigned long long* status = reinterpret_cast<unsigned long long*>(scratch + kStatusOffset);
     if (threadIdx.x == 0) *status = bad;
     if (bad != ~0ull) return;
-    const int64_t m = (int64_t)n * n;
-    double* rr = V.cg[1];
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) rr[k] = r[k];
+    const PLvl<double>& L = V.lv[0];
+    const int np = L.np, m2 = np * (np / 2);
+    for (int k = threadIdx.x; k < n * n; k += blockDim.x) V.r[k / n * np + k % n] = r[k];
     __syncthreads();
-    block_precondition<double>(A, V, rr, V.cg[4], red);
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) z[k] = V.cg[4][k];
+    for (int q = threadIdx.x; q < m2; q += blockDim.x) pair_start_cycle<double>(L, q, load_pair(V.r + 2 * q));
+    __syncthreads();
+    block_precondition<double>(A, V, red);
+    for (int k = threadIdx.x; k < n * n; k += blockDim.x) z[k] = L.x[k / n * np + k % n];
 }
 
 // Device address of the scratch array in the current device's context. It is

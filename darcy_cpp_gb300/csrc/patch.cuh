@@ -1,0 +1,466 @@
+// Level operations of the block engine (one CTA, one problem) on a padded
+// layout, two cells of a colour at a time.
+//
+// A level of side n is stored with side np = 2 nc, nc = (n + 1) / 2: an even
+// pitch, so that rows and pairs are 8- / 16-byte aligned for every n, and
+// whole 2 x 2 aggregates ("patches"), so that one index serves the four cells
+// of a patch and its coarse cell. Cells outside the domain (the last row and
+// column of an odd side) hold zero coefficients and stay zero. Once the next
+// coarser level is built, the faces on the domain's east and north boundary
+// are set to zero, and nf has np zeros and e two zeros before the array, x
+// np zeros before and after it: a neighbour outside the domain then enters as
+// 0 * (some finite number), which leaves the sum as the reference's skipped
+// term does, and no pass tests for a boundary.
+//
+// Why patches: the earlier passes walked the cells of one colour with an
+// integer division, four boundary tests and ten scalar loads a cell; a
+// 64 x 64 problem took ~120 thousand warp instructions an iteration and the
+// scheduler had nothing to issue 58% (FP32 cycle) to 78% (FP64) of the time.
+#pragma once
+
+#include "common.cuh"
+
+namespace dgpu {
+
+template <class T>
+struct PLvl {
+    int n, nc, np;
+    unsigned rcp;  // ceil(2^32 / nc) while the product below is exact, else 0
+    const T* e;
+    const T* nf;
+    const T* d;
+    const T* id;
+    T* x;
+    T* b;
+};
+
+template <class T>
+struct Pair;
+template <>
+struct Pair<float> {
+    using type = float2;
+};
+template <>
+struct Pair<double> {
+    using type = double2;
+};
+template <class T>
+using Pair_t = typename Pair<T>::type;
+
+template <class T>
+__device__ __forceinline__ Pair_t<T> load_pair(const T* p) {
+    return *reinterpret_cast<const Pair_t<T>*>(p);
+}
+
+// q / nc for q < 2 nc^2 (pairs of a level) as the high half of a product:
+// exact while 2 nc^3 < 2^32.
+__host__ __device__ inline unsigned row_reciprocal(int nc) {
+    return nc >= 2 && nc <= 1280 ? (unsigned)((0x100000000ull + (unsigned)nc - 1) / (unsigned)nc) : 0u;
+}
+__device__ __forceinline__ int patch_row(int q, int nc, unsigned rcp) {
+    return rcp ? (int)__umulhi((unsigned)q, rcp) : q / nc;
+}
+
+// The passes below work on one patch whose first cell is k = 2 I np + 2 J.
+// Colour 0 holds the cells (0, 0) and (1, 1) of a patch, colour 1 the cells
+// (0, 1) and (1, 0). Terms in the order of include/darcy/level.hpp:105-161.
+
+// Colour 0 from a zero iterate: x = b / d.
+template <class T>
+__device__ __forceinline__ void patch_red_zero(const PLvl<T>& L, T* x, const T* b, int k) {
+    const int k1 = k + L.np + 1;
+    const T v0 = b[k] * L.id[k], v1 = b[k1] * L.id[k1];
+    x[k] = v0;
+    x[k1] = v1;
+}
+
+template <class T>
+__device__ __forceinline__ void patch_red(const PLvl<T>& L, const T* x, const T* b, int k, T& o0, T& o1) {
+    const int np = L.np, k1 = k + np + 1;
+    const T x01 = x[k + 1], x10 = x[k + np];
+    const Pair_t<T> n0 = load_pair(L.nf + k), e1 = load_pair(L.e + k + np);
+    T v0 = b[k], v1 = b[k1];
+    v0 += L.e[k] * x01;
+    v1 += e1.y * x[k1 + 1];
+    v0 += L.e[k - 1] * x[k - 1];
+    v1 += e1.x * x10;
+    v0 += n0.x * x10;
+    v1 += L.nf[k1] * x[k1 + np];
+    v0 += L.nf[k - np] * x[k - np];
+    v1 += n0.y * x01;
+    o0 = v0 * L.id[k];
+    o1 = v1 * L.id[k1];
+}
+
+template <class T>
+__device__ __forceinline__ void patch_black(const PLvl<T>& L, const T* x, const T* b, int k, T& o0, T& o1) {
+    const int np = L.np, kb = k + 1, kc = k + np;
+    const T x00 = x[k], x11 = x[kc + 1];
+    const Pair_t<T> n0 = load_pair(L.nf + k), e0 = load_pair(L.e + k);
+    T v0 = b[kb], v1 = b[kc];
+    v0 += e0.y * x[kb + 1];
+    v1 += L.e[kc] * x11;
+    v0 += e0.x * x00;
+    v1 += L.e[kc - 1] * x[kc - 1];
+    v0 += n0.y * x11;
+    v1 += L.nf[kc] * x[kc + np];
+    v0 += L.nf[kb - np] * x[kb - np];
+    v1 += n0.x * x00;
+    o0 = v0 * L.id[kb];
+    o1 = v1 * L.id[kc];
+}
+
+// Colour 1 seeing colour 0 through the prolongation x + P xc. The colour-0
+// pass that follows overwrites every colour-0 cell and colour 1 never reads
+// its own value, so the corrected iterate is not stored (level.hpp:230-237
+// followed by :145-161).
+template <class T>
+__device__ __forceinline__ void patch_black_prolong(const PLvl<T>& L, const T* x, const T* b, int k,
+                                                    const T* xc, int K, int npc, T& o0, T& o1) {
+    const int np = L.np, kb = k + 1, kc = k + np;
+    const T c = xc[K];
+    const T x00 = x[k] + c, x11 = x[kc + 1] + c;
+    const Pair_t<T> n0 = load_pair(L.nf + k), e0 = load_pair(L.e + k);
+    T v0 = b[kb], v1 = b[kc];
+    v0 += e0.y * (x[kb + 1] + xc[K + 1]);
+    v1 += L.e[kc] * x11;
+    v0 += e0.x * x00;
+    v1 += L.e[kc - 1] * (x[kc - 1] + xc[K - 1]);
+    v0 += n0.y * x11;
+    v1 += L.nf[kc] * (x[kc + np] + xc[K + npc]);
+    v0 += L.nf[kb - np] * (x[kb - np] + xc[K - npc]);
+    v1 += n0.x * x00;
+    o0 = v0 * L.id[kb];
+    o1 = v1 * L.id[kc];
+}
+
+// Sum of b - A x over the patch, cells in row-major order (level.hpp:122-137,
+// :214-227).
+template <class T>
+__device__ __forceinline__ T patch_residual(const PLvl<T>& L, const T* x, const T* b, int k) {
+    const int np = L.np, k1 = k + np;
+    const Pair_t<T> x0 = load_pair(x + k), x1 = load_pair(x + k1), xn = load_pair(x + k1 + np),
+                    xs = load_pair(x + k - np);
+    const Pair_t<T> e0 = load_pair(L.e + k), e1 = load_pair(L.e + k1);
+    const Pair_t<T> n0 = load_pair(L.nf + k), n1 = load_pair(L.nf + k1), ns = load_pair(L.nf + k - np);
+    const Pair_t<T> d0 = load_pair(L.d + k), d1 = load_pair(L.d + k1), b0 = load_pair(b + k), b1 = load_pair(b + k1);
+    T v = d0.x * x0.x;
+    v -= e0.x * x0.y;
+    v -= L.e[k - 1] * x[k - 1];
+    v -= n0.x * x1.x;
+    v -= ns.x * xs.x;
+    T s = b0.x - v;
+    v = d0.y * x0.y;
+    v -= e0.y * x[k + 2];
+    v -= e0.x * x0.x;
+    v -= n0.y * x1.y;
+    v -= ns.y * xs.y;
+    s += b0.y - v;
+    v = d1.x * x1.x;
+    v -= e1.x * x1.y;
+    v -= L.e[k1 - 1] * x[k1 - 1];
+    v -= n1.x * xn.x;
+    v -= n0.x * x0.x;
+    s += b1.x - v;
+    v = d1.y * x1.y;
+    v -= e1.y * x[k1 + 2];
+    v -= e1.x * x1.x;
+    v -= n1.y * xn.y;
+    v -= n0.y * x0.y;
+    s += b1.y - v;
+    return s;
+}
+
+// ------------------------------------------------------------ CTA passes
+//
+// kU patches of a thread are computed before any of them is stored, so that
+// their loads are in flight together (an FP32 patch needs 16-18 values, an
+// FP64 one twice the registers).
+
+template <class T>
+constexpr int kPatchUnroll = sizeof(T) == 4 ? 1 : 1;
+
+template <class T>
+__device__ __forceinline__ void pass_red_zero(const PLvl<T>& L) {
+    const int nc = L.nc, cnt = nc * nc;
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x)
+        patch_red_zero(L, L.x, L.b, 2 * q + 2 * patch_row(q, nc, L.rcp) * nc);
+}
+
+template <class T, int kColour>
+__device__ __forceinline__ void pass_colour(const PLvl<T>& L) {
+    constexpr int kU = kPatchUnroll<T>;
+    const int nc = L.nc, cnt = nc * nc, np = L.np;
+    const unsigned rcp = L.rcp;
+    for (int q0 = threadIdx.x; q0 < cnt; q0 += kU * blockDim.x) {
+        T o0[kU], o1[kU];
+        int kk[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * blockDim.x;
+            if (u > 0 && q >= cnt) break;
+            kk[u] = 2 * q + 2 * patch_row(q, nc, rcp) * nc;
+            if (kColour == 0)
+                patch_red(L, L.x, L.b, kk[u], o0[u], o1[u]);
+            else
+                patch_black(L, L.x, L.b, kk[u], o0[u], o1[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (u > 0 && q0 + u * (int)blockDim.x >= cnt) break;
+            L.x[kk[u] + (kColour == 0 ? 0 : 1)] = o0[u];
+            L.x[kk[u] + (kColour == 0 ? np + 1 : np)] = o1[u];
+        }
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void pass_black_prolong(const PLvl<T>& L, const PLvl<T>& C) {
+    constexpr int kU = kPatchUnroll<T>;
+    const int nc = L.nc, cnt = nc * nc, np = L.np, npc = C.np;
+    const unsigned rcp = L.rcp;
+    for (int q0 = threadIdx.x; q0 < cnt; q0 += kU * blockDim.x) {
+        T o0[kU], o1[kU];
+        int kk[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int q = q0 + u * blockDim.x;
+            if (u > 0 && q >= cnt) break;
+            const int I = patch_row(q, nc, rcp);
+            kk[u] = 2 * q + 2 * I * nc;
+            patch_black_prolong(L, L.x, L.b, kk[u], C.x, q + I * (npc - nc), npc, o0[u], o1[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            if (u > 0 && q0 + u * (int)blockDim.x >= cnt) break;
+            L.x[kk[u] + 1] = o0[u];
+            L.x[kk[u] + np] = o1[u];
+        }
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void pass_residual_restrict(const PLvl<T>& L, const PLvl<T>& C) {
+    const int nc = L.nc, cnt = nc * nc, npc = C.np;
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+        const int I = patch_row(q, nc, L.rcp);
+        C.b[q + I * (npc - nc)] = patch_residual(L, L.x, L.b, 2 * q + 2 * I * nc);
+    }
+}
+
+// x = Tt b for the dense tail operator (N x N, N the padded cells of the
+// tail's first level, rows `pitch` apart): four lanes a row, each taking
+// every fourth 16-byte vector of it. With rows 64 bytes past a multiple of
+// 128 apart, the eight lanes of a quarter warp (two rows) read distinct banks.
+// One warp a row, two elements a lane, spent its time in the five dependent
+// shuffles of each row's sum.
+template <class T>
+__host__ __device__ inline int tail_pitch(int N) {
+    const int bytes = N * (int)sizeof(T);
+    return (int)(((bytes + 63) / 128 * 128 + 64) / sizeof(T));
+}
+template <class T>
+__device__ __forceinline__ void block_matvec(const T* __restrict__ Tt, int N, int pitch, const T* b, T* x) {
+    constexpr int kW = 16 / sizeof(T);
+    const int lane4 = threadIdx.x & 3;
+    for (int t = threadIdx.x; (t & ~31) < 4 * N; t += blockDim.x) {
+        const int row = t >> 2;
+        T acc = T(0);
+        if (row < N) {
+            const T* Tr = Tt + row * pitch;
+#pragma unroll 4
+            for (int c = lane4 * kW; c < N; c += 4 * kW) {
+                if constexpr (sizeof(T) == 4) {
+                    const float4 m = *reinterpret_cast<const float4*>(Tr + c), v = *reinterpret_cast<const float4*>(b + c);
+                    acc += m.x * v.x;
+                    acc += m.y * v.y;
+                    acc += m.z * v.z;
+                    acc += m.w * v.w;
+                } else {
+                    const double2 m = *reinterpret_cast<const double2*>(Tr + c),
+                                  v = *reinterpret_cast<const double2*>(b + c);
+                    acc += m.x * v.x;
+                    acc += m.y * v.y;
+                }
+            }
+        }
+        acc += __shfl_down_sync(0xffffffffu, acc, 2, 4);
+        acc += __shfl_down_sync(0xffffffffu, acc, 1, 4);
+        if (row < N && lane4 == 0) x[row] = acc;
+    }
+}
+
+// ------------------------------------------------------------ the cycle
+//
+// One cycle at level 0 (include/darcy/multigrid.hpp:88-127, the recursion
+// unrolled into two bits of remaining calls a level) without its first
+// colour-0 pass from zero and without its last colour-0 pass: the caller
+// merges those into the loops that produce b and consume x. The levels from
+// tl down are the dense operator Tt ("x = 0, then gamma cycles"); with Tt ==
+// null they are visited down to the 1 x 1 level, solved exactly (with the
+// FP64 reciprocal diagonal id64 in the FP32 cycle). At least two levels.
+//
+// A level's second call starts where its first ended: that call's last
+// colour-0 pass reads the same colour-1 values as the second call's first
+// would, so the latter is skipped (same bits).
+template <class T>
+__device__ void patch_cycle(const PLvl<T>* lv, int nlev, int pre, int post, int gamma, const double* id64,
+                            const T* Tt, int tl) {
+    unsigned long long calls = 1;  // remaining calls, two bits a level
+    int l = 0;
+    bool zero = true;              // the level's iterate is zero (its first call)
+    const int last = Tt ? tl - 1 : nlev - 2;  // deepest level that is smoothed
+    auto descend = [&](int lvl) {
+        const PLvl<T>& A = lv[lvl];
+        if (zero && lvl > 0) {
+            pass_red_zero(A);
+            __syncthreads();
+        }
+        pass_colour<T, 1>(A);
+        __syncthreads();
+        for (int s = 1; s < pre; ++s) {
+            pass_colour<T, 0>(A);
+            __syncthreads();
+            pass_colour<T, 1>(A);
+            __syncthreads();
+        }
+        pass_residual_restrict(A, lv[lvl + 1]);
+        __syncthreads();
+    };
+    auto ascend = [&](int lvl) {
+        const PLvl<T>& A = lv[lvl];
+        pass_black_prolong(A, lv[lvl + 1]);
+        __syncthreads();
+        for (int s = 1; s < post; ++s) {
+            pass_colour<T, 0>(A);
+            __syncthreads();
+            pass_colour<T, 1>(A);
+            __syncthreads();
+        }
+        if (lvl > 0) {
+            pass_colour<T, 0>(A);
+            __syncthreads();
+        }
+    };
+    for (;;) {
+        while (l < last) {
+            descend(l);
+            ++l;
+            calls = (calls & ~(3ull << (2 * l))) | ((unsigned long long)gamma << (2 * l));
+            zero = true;
+        }
+        descend(l);
+        if (Tt) {
+            const PLvl<T>& B = lv[tl];
+            const int N = B.np * B.np;
+            block_matvec<T>(Tt, N, tail_pitch<T>(N), B.b, B.x);
+        } else if (threadIdx.x == 0) {  // the 1 x 1 level; a second call finds its exact solution again
+            const PLvl<T>& B = lv[nlev - 1];
+            B.x[0] = id64 ? (T)((double)B.b[0] * id64[0]) : B.b[0] * B.id[0];
+        }
+        __syncthreads();
+        ascend(l);
+        for (;;) {
+            calls -= 1ull << (2 * l);
+            if ((calls >> (2 * l)) & 3ull) break;  // run this level's cycle again
+            if (l == 0) return;
+            --l;
+            ascend(l);
+        }
+        zero = false;
+    }
+}
+
+// -------------------------------------------------- many right-hand sides
+//
+// The recursion below level `l0` for `nrhs` right-hand sides at once (gamma
+// calls from zero at l0), used to build the dense tail. Right-hand side r of
+// a level is at x + r * stride, b + r * stride, stride = np^2 + 2 np.
+
+__host__ __device__ inline int rhs_stride(int np) { return np * np + 2 * np; }
+
+template <class T, class F>
+__device__ __forceinline__ void for_patches_m(const PLvl<T>& L, int nrhs, F&& f) {
+    const int nc = L.nc, per = nc * nc, st = rhs_stride(L.np);
+    for (int t = threadIdx.x; t < per * nrhs; t += blockDim.x) {
+        const int r = t / per, q = t - r * per;
+        const int I = patch_row(q, nc, L.rcp);
+        f(L.x + r * st, L.b + r * st, r, 2 * q + 2 * I * nc, q, I);
+    }
+    __syncthreads();
+}
+
+template <class T>
+__device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int post, int gamma, int nrhs,
+                              const double* id64) {
+    unsigned long long calls = (unsigned long long)gamma << (2 * l0);
+    int l = l0;
+    bool zero = true;
+    auto red = [&](const PLvl<T>& A) {
+        for_patches_m(A, nrhs, [&](T* x, const T* b, int, int k, int, int) {
+            T o0, o1;
+            patch_red(A, x, b, k, o0, o1);
+            x[k] = o0;
+            x[k + A.np + 1] = o1;
+        });
+    };
+    auto black = [&](const PLvl<T>& A) {
+        for_patches_m(A, nrhs, [&](T* x, const T* b, int, int k, int, int) {
+            T o0, o1;
+            patch_black(A, x, b, k, o0, o1);
+            x[k + 1] = o0;
+            x[k + A.np] = o1;
+        });
+    };
+    for (;;) {
+        while (l + 1 < nlev) {
+            const PLvl<T>& A = lv[l];
+            const PLvl<T>& C = lv[l + 1];
+            const int stc = rhs_stride(C.np), npc = C.np;
+            if (zero)
+                for_patches_m(A, nrhs, [&](T* x, const T* b, int, int k, int, int) { patch_red_zero(A, x, b, k); });
+            black(A);
+            for (int s = 1; s < pre; ++s) {
+                red(A);
+                black(A);
+            }
+            for_patches_m(A, nrhs, [&](T* x, const T* b, int r, int k, int q, int I) {
+                C.b[r * stc + q + I * (npc - A.nc)] = patch_residual(A, x, b, k);
+            });
+            ++l;
+            calls = (calls & ~(3ull << (2 * l))) | ((unsigned long long)gamma << (2 * l));
+            zero = true;
+        }
+        {  // the 1 x 1 level
+            const PLvl<T>& A = lv[l];
+            const int st = rhs_stride(A.np);
+            for (int r = threadIdx.x; r < nrhs; r += blockDim.x)
+                A.x[r * st] = id64 ? (T)((double)A.b[r * st] * id64[0]) : A.b[r * st] * A.id[0];
+            __syncthreads();
+            calls &= ~(3ull << (2 * l));  // further calls of it change nothing
+        }
+        for (;;) {
+            if (((calls >> (2 * l)) & 3ull) != 0) calls -= 1ull << (2 * l);
+            if (l + 1 < nlev && ((calls >> (2 * l)) & 3ull) != 0) break;
+            if (l == l0) return;
+            --l;
+            const PLvl<T>& A = lv[l];
+            const PLvl<T>& C = lv[l + 1];
+            const int stc = rhs_stride(C.np), npc = C.np;
+            for_patches_m(A, nrhs, [&](T* x, const T* b, int r, int k, int q, int I) {
+                T o0, o1;
+                patch_black_prolong(A, x, b, k, C.x + r * stc, q + I * (npc - A.nc), npc, o0, o1);
+                x[k + 1] = o0;
+                x[k + A.np] = o1;
+            });
+            for (int s = 1; s < post; ++s) {
+                red(A);
+                black(A);
+            }
+            red(A);
+        }
+        zero = false;
+    }
+}
+
+}  // namespace dgpu

@@ -49,46 +49,12 @@ __device__ __forceinline__ void build_fine(const double* __restrict__ a, const L
     }
 }
 
-// build_fine for one CTA with every face computed once (one division per
-// face instead of two; FP64 division is tens of instructions on the narrow
-// FP64 pipe): the east/north faces and the boundary faces first, then the
-// diagonal from the stored faces in build_fine's summation order. A cell's
-// west/south face is its neighbour's east/north face, the same bits since
-// harmonic() is symmetric, so the level equals build_fine's bit for bit.
-// with_id false leaves id unwritten (the FP32 cycle computes its own
-// reciprocal from the FP32 diagonal). Returns with the CTA synchronised.
-__device__ __forceinline__ void build_fine_block(const double* __restrict__ a, const Lvl64& L,
-                                                 unsigned long long* bad, bool with_id) {
-    const int n = L.n;
-    const int64_t m = (int64_t)n * n;
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-        const int i = (int)(k / n), j = (int)(k - (int64_t)i * n);
-        const double c = a[k];
-        if (!(c > 0.0) || !isfinite(c)) atomicMin(bad, (unsigned long long)k);
-        L.e[k] = (j + 1 < n) ? harmonic(c, a[k + 1]) : c;
-        L.nf[k] = (i + 1 < n) ? harmonic(c, a[k + n]) : c;
-        if (j == 0) L.wb[i] = c;
-        if (i == 0) L.sb[j] = c;
-    }
-    __syncthreads();
-    for (int64_t k = threadIdx.x; k < m; k += blockDim.x) {
-        const int i = (int)(k / n), j = (int)(k - (int64_t)i * n);
-        const double w = (j > 0) ? L.e[k - 1] : L.wb[i];
-        const double s = (i > 0) ? L.nf[k - n] : L.sb[j];
-        const double dd = L.e[k] + w + L.nf[k] + s;
-        L.d[k] = dd;
-        if (with_id) L.id[k] = 1.0 / dd;
-    }
-    __syncthreads();
-}
-
 // Galerkin coarse operator P^T A P by face summation (level.hpp:171-211),
 // including the width-one trailing aggregate of an odd grid. West/south fine
 // faces come from the neighbour's east/north face (same bits) or, on the
-// domain boundary, from wb/sb; summation order is the reference's. with_id
-// false leaves id unwritten, as in build_fine_block.
+// domain boundary, from wb/sb; summation order is the reference's.
 template <class S>
-__device__ __forceinline__ void coarsen(const Lvl64& F, const Lvl64& C, bool with_id = true) {
+__device__ __forceinline__ void coarsen(const Lvl64& F, const Lvl64& C) {
     const int n = F.n, nc = C.n;
     const int64_t mc = (int64_t)nc * nc;
     for (int64_t K = S::start(); K < mc; K += S::stride()) {
@@ -108,7 +74,7 @@ __device__ __forceinline__ void coarsen(const Lvl64& F, const Lvl64& C, bool wit
         C.e[K] = ce;
         C.nf[K] = cn;
         C.d[K] = dd;
-        if (with_id) C.id[K] = 1.0 / dd;
+        C.id[K] = 1.0 / dd;
         if (J == 0) C.wb[I] = cw;
         if (I == 0) C.sb[J] = cs;
     }

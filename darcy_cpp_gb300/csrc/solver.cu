@@ -74,6 +74,8 @@ constexpr int kTailSide = 32;
 // 16384 x 128^2 + 64 x 512^2 end to end, 1.64 / 1.29 s with the 512^2
 // problems in the block launch against 1.49-1.62 / 1.10 s routed.
 constexpr int kGridEngineMinSide = 384;
+// The block engine's cell index is a 32-bit int.
+constexpr int kBlockEngineMaxSide = 16384;
 // Grid-engine levels of at least this side run the unfused kernels (see
 // emit_visit_hybrid); smaller ones the fused visits. Measured on GB300
 // (mixed / FP64, ms per solve, all-fused -> unfused from this side):
@@ -853,11 +855,12 @@ void grid_solve(dgpu_context* C, const double* a, const double* f, double fscala
 }
 
 // Whether a batched problem of side n goes to the grid engine, in a batch of
-// total_cells cells. DARCY_GPU_GRID_SIDE=s overrides: side >= s, nothing else.
+// total_cells cells. DARCY_GPU_GRID_SIDE=s overrides: side >= s
+// (or beyond the block engine's index).
 bool route_to_grid(const dgpu_context* C, int64_t n, int64_t total_cells) {
     const char* e = std::getenv("DARCY_GPU_GRID_SIDE");
     const int v = e ? std::atoi(e) : 0;
-    if (v >= 1) return n >= v;
+    if (v >= 1) return n >= v || n > kBlockEngineMaxSide;
     (void)C;
     (void)total_cells;
     return n >= kGridEngineMinSide;
