@@ -364,8 +364,10 @@ __device__ __forceinline__ double2 pair_apply(const Lvl64& L, const double* __re
     return make_double2(v0, v1);
 }
 
-// y = A x over a block, FP64, returning sum x . y.
-__device__ __forceinline__ double block_apply_dot(const Lvl64& L, const double* x, double* y, double* red) {
+// y = A x over a block, FP64, returning then(sum x . y).
+template <class F>
+__device__ __forceinline__ double block_apply_dot(const Lvl64& L, const double* x, double* y, double* red,
+                                                  F&& then) {
     const int n2 = (L.n + 1) / 2, m2 = 2 * n2 * n2;
     double acc = 0.0;
     for (int q = threadIdx.x; q < m2; q += blockDim.x) {
@@ -375,7 +377,7 @@ __device__ __forceinline__ double block_apply_dot(const Lvl64& L, const double* 
         acc += xc.x * v.x;
         acc += xc.y * v.y;
     }
-    return block_sum_wide(acc, red);
+    return block_sum_then(acc, red, then);
 }
 
 // b = r in the cycle's precision and the cycle's first pass (colour 0 from a
@@ -394,10 +396,10 @@ __device__ __forceinline__ void pair_start_cycle(const PLvl<T>& L, int q, double
 }
 
 // z = M r for one problem, r already handed over by pair_start_cycle on every
-// pair (multigrid) and the CTA synchronised since; returns r . z. The
+// pair (multigrid) and the CTA synchronised since; returns then(r . z). The
 // cycle's iterate lv[0].x is z, in the cycle's precision.
-template <class T>
-__device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V, double* red) {
+template <class T, class F>
+__device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V, double* red, F&& then) {
     const PLvl<T>& L = V.lv[0];
     const double* r = V.r;
     double acc = 0.0;
@@ -433,7 +435,7 @@ __device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V,
             acc += r[k] * zk;
         }
     }
-    return block_sum_wide(acc, red);
+    return block_sum_then(acc, red, then);
 }
 
 // The dense tail of one problem: column j = the tail map applied to e_j, all

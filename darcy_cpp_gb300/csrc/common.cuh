@@ -280,7 +280,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 // shuffle tree: blockDim/32 + 4 full-warp adds per block instead of
 // 5 blockDim/32 + 5. `scratch` holds blockDim.x doubles; blockDim.x is a
 // multiple of 32. Fixed order; every thread gets the total.
-__device__ __forceinline__ double block_sum_wide(double v, double* scratch) {
+//
+// `then(total)` runs in warp 0 alone (its lane 0's value counts) and its
+// result is what every thread gets: a division or square root of the total
+// costs tens of FP64 instructions a warp, and evaluated by every warp of a CTA
+// the solvers' three divisions and one square root an iteration took a
+// quarter of the FP64 pipe's time (64^2, FP32 cycle, 256 threads).
+template <class F>
+__device__ __forceinline__ double block_sum_then(double v, double* scratch, F&& then) {
     const int t = threadIdx.x, nw = (int)(blockDim.x >> 5);
     __syncthreads();  // the previous call's readers are done with scratch
     scratch[t] = v;
@@ -291,11 +298,14 @@ __device__ __forceinline__ double block_sum_wide(double v, double* scratch) {
             s0 += scratch[t + 32 * w];
             if (w + 1 < nw) s1 += scratch[t + 32 * (w + 1)];
         }
-        const double s = warp_sum(s0 + s1);
+        const double s = then(warp_sum(s0 + s1));
         if (t == 0) scratch[0] = s;
     }
     __syncthreads();
     return scratch[0];
+}
+__device__ __forceinline__ double block_sum_wide(double v, double* scratch) {
+    return block_sum_then(v, scratch, [](double s) { return s; });
 }
 
 // Grid-wide deterministic sum: each block stores its partial, the last block

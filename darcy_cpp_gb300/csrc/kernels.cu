@@ -947,6 +947,8 @@ size_t block_arena_bytes(int n, bool mixed, size_t sbudget) {
 template <class T>
 __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>& V, double* red,
                                 unsigned long long* s_bad) {
+    __shared__ double s_rz;
+    __shared__ bool s_broke;
     const int n = A.side[pid];
     const int64_t off = A.off[pid];
     double *r = V.r, *p = V.p, *ap = V.ap, *u = V.u;
@@ -984,7 +986,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         u[c] = u0 ? u0[k] : 0.0;
         sb += bk * bk;
     }
-    const double bnorm = sqrt(block_sum_wide(sb, red));
+    const double bnorm = block_sum_then(sb, red, [](double t) { return sqrt(t); });
     int iterations = 0, converged = 0;
     bool sound = true;
     double residual = 0.0;
@@ -1015,7 +1017,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             sbu += bb.x * uu.x;
             sbu += bb.y * uu.y;
         }
-        residual = sqrt(block_sum_wide(sr, red)) / bnorm;
+        residual = block_sum_then(sr, red, [&](double t) { return sqrt(t) / bnorm; });
         if (A.u0_fallback) bu0 = block_sum_wide(sbu, red);
     }
     if (record && threadIdx.x == 0) A.history[0] = residual;
@@ -1030,7 +1032,8 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     } else {
         __syncthreads();
         start_cycle();
-        double rz = block_precondition<T>(A, V, red);
+        auto itself = [](double t) { return t; };
+        double rz = block_precondition<T>(A, V, red, itself);
         // A predicted start no better than zero is dropped for the zero start,
         // the fallback it is judged against. CG minimises the error's energy
         // norm; r0 . M r0 (the first preconditioned residual, computed here
@@ -1046,8 +1049,9 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             residual = 1.0;
             __syncthreads();
             start_cycle();
-            rz = block_precondition<T>(A, V, red);
+            rz = block_precondition<T>(A, V, red, itself);
         }
+        if (threadIdx.x == 0) s_rz = rz;  // r . z of the current direction (thread 0's)
         double beta = 0.0;
         for (int it = 0; it < A.max_iter; ++it) {
             // p = z + beta p (z alone before the first iteration)
@@ -1062,14 +1066,17 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
                 reinterpret_cast<double2*>(p)[q] = pp;
             }
             __syncthreads();
-            const double pap = block_apply_dot(h0, p, ap, red);
-            if (!(fabs(pap) > 0.0) || !isfinite(pap)) {
+            // alpha = rz / (p . Ap), or a breakdown (solver.hpp:149-155)
+            const double alpha = block_apply_dot(h0, p, ap, red, [&](double pap) {
+                if (threadIdx.x == 0) s_broke = !(fabs(pap) > 0.0) || !isfinite(pap);
+                return s_rz / pap;
+            });
+            if (s_broke) {
                 iterations = it;
                 converged = 0;
                 sound = false;
                 break;
             }
-            const double alpha = rz / pap;
             double rr = 0.0;
             for (int q = threadIdx.x; q < m2; q += blockDim.x) {
                 double2 uu = load_pair(u + 2 * q), rv = load_pair(r + 2 * q);
@@ -1084,16 +1091,19 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
                 rr += rv.y * rv.y;
                 if (mg) pair_start_cycle<T>(L0, q, rv);
             }
-            residual = sqrt(block_sum_wide(rr, red)) / bnorm;
+            residual = block_sum_then(rr, red, [&](double t) { return sqrt(t) / bnorm; });
             iterations = it + 1;
             if (record && threadIdx.x == 0) A.history[it + 1] = residual;
             if (residual < A.tol) {
                 converged = 1;
                 break;
             }
-            const double rz_new = block_precondition<T>(A, V, red);
-            beta = rz_new / rz;
-            rz = rz_new;
+            beta = block_precondition<T>(A, V, red, [&](double t) {
+                const double ratio = t / s_rz;
+                __syncwarp();
+                if (threadIdx.x == 0) s_rz = t;
+                return ratio;
+            });
         }
     }
 
@@ -1115,7 +1125,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
                 }
             }
         }
-        true_res = sqrt(block_sum_wide(tr, red)) / bnorm;
+        true_res = block_sum_then(tr, red, [&](double t) { return sqrt(t) / bnorm; });
     }
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
         const int i = k / n;

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) k_precondition_noalloc(unsigned char* scr
     __syncthreads();
     for (int q = threadIdx.x; q < m2; q += blockDim.x) pair_start_cycle<double>(L, q, load_pair(V.r + 2 * q));
     __syncthreads();
-    block_precondition<double>(A, V, red);
+    block_precondition<double>(A, V, red, [](double rz) { return rz; });
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) z[k] = L.x[k / n * np + k % n];
 }
 

@@ -134,51 +134,46 @@ __device__ __forceinline__ void patch_black_prolong(const PLvl<T>& L, const T* x
     o1 = v1 * L.id[kc];
 }
 
-// Sum of b - A x over the patch, cells in row-major order (level.hpp:122-137,
-// :214-227).
-template <class T>
+// Sum of b - A x over the patch (level.hpp:122-137, :214-227) after a
+// colour-1 pass. That pass has just solved the colour-1 cells' equations, so
+// their residual is zero (up to the rounding of the very values it would be
+// computed from) and only the two colour-0 cells contribute: half the
+// arithmetic and none of the loads of colour 1's d and b.
+//
+// kFromZero: the colour-0 values come from the pass x = b / d on a zero
+// iterate, so b - d x is zero too (again up to rounding) and what is left is
+// the flow from the colour-1 neighbours. (FP64, where the pipe is 88% busy:
+// 27 operations a patch become 9 or 13; 1024 x 64^2 8.25 -> 6.97 ms, 512 x
+// 128^2 30.9 -> 26.8 ms; iteration counts within +-0.1 on average in both
+// forms at contrasts 4 to 1e6.)
+template <class T, bool kFromZero>
 __device__ __forceinline__ T patch_residual(const PLvl<T>& L, const T* x, const T* b, int k) {
-    const int np = L.np, k1 = k + np;
-    const Pair_t<T> x0 = load_pair(x + k), x1 = load_pair(x + k1), xn = load_pair(x + k1 + np),
-                    xs = load_pair(x + k - np);
-    const Pair_t<T> e0 = load_pair(L.e + k), e1 = load_pair(L.e + k1);
-    const Pair_t<T> n0 = load_pair(L.nf + k), n1 = load_pair(L.nf + k1), ns = load_pair(L.nf + k - np);
-    const Pair_t<T> d0 = load_pair(L.d + k), d1 = load_pair(L.d + k1), b0 = load_pair(b + k), b1 = load_pair(b + k1);
-    T v = d0.x * x0.x;
-    v -= e0.x * x0.y;
-    v -= L.e[k - 1] * x[k - 1];
-    v -= n0.x * x1.x;
-    v -= ns.x * xs.x;
-    T s = b0.x - v;
-    v = d0.y * x0.y;
-    v -= e0.y * x[k + 2];
-    v -= e0.x * x0.x;
-    v -= n0.y * x1.y;
-    v -= ns.y * xs.y;
-    s += b0.y - v;
-    v = d1.x * x1.x;
-    v -= e1.x * x1.y;
-    v -= L.e[k1 - 1] * x[k1 - 1];
-    v -= n1.x * xn.x;
-    v -= n0.x * x0.x;
-    s += b1.x - v;
-    v = d1.y * x1.y;
-    v -= e1.y * x[k1 + 2];
-    v -= e1.x * x1.x;
-    v -= n1.y * xn.y;
-    v -= n0.y * x0.y;
-    s += b1.y - v;
-    return s;
+    const int np = L.np, k1 = k + np + 1;
+    const T x01 = x[k + 1], x10 = x[k + np];
+    const Pair_t<T> n0 = load_pair(L.nf + k), e1 = load_pair(L.e + k + np);
+    T v0, v1;
+    if (kFromZero) {
+        v0 = L.e[k] * x01;
+        v1 = e1.y * x[k1 + 1];
+    } else {
+        v0 = b[k] - L.d[k] * x[k];
+        v1 = b[k1] - L.d[k1] * x[k1];
+        v0 += L.e[k] * x01;
+        v1 += e1.y * x[k1 + 1];
+    }
+    v0 += L.e[k - 1] * x[k - 1];
+    v1 += e1.x * x10;
+    v0 += n0.x * x10;
+    v1 += L.nf[k1] * x[k1 + np];
+    v0 += L.nf[k - np] * x[k - np];
+    v1 += n0.y * x01;
+    return v0 + v1;
 }
 
 // ------------------------------------------------------------ CTA passes
 //
-// kU patches of a thread are computed before any of them is stored, so that
-// their loads are in flight together (an FP32 patch needs 16-18 values, an
-// FP64 one twice the registers).
-
-template <class T>
-constexpr int kPatchUnroll = sizeof(T) == 4 ? 1 : 1;
+// (Two patches of a thread at once, all loads before the first store, measured
+// slower: 4096 x 64^2 mixed 13.2 -> 13.8 ms at 256 threads and 32 KiB.)
 
 template <class T>
 __device__ __forceinline__ void pass_red_zero(const PLvl<T>& L) {
@@ -189,62 +184,37 @@ __device__ __forceinline__ void pass_red_zero(const PLvl<T>& L) {
 
 template <class T, int kColour>
 __device__ __forceinline__ void pass_colour(const PLvl<T>& L) {
-    constexpr int kU = kPatchUnroll<T>;
     const int nc = L.nc, cnt = nc * nc, np = L.np;
-    const unsigned rcp = L.rcp;
-    for (int q0 = threadIdx.x; q0 < cnt; q0 += kU * blockDim.x) {
-        T o0[kU], o1[kU];
-        int kk[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int q = q0 + u * blockDim.x;
-            if (u > 0 && q >= cnt) break;
-            kk[u] = 2 * q + 2 * patch_row(q, nc, rcp) * nc;
-            if (kColour == 0)
-                patch_red(L, L.x, L.b, kk[u], o0[u], o1[u]);
-            else
-                patch_black(L, L.x, L.b, kk[u], o0[u], o1[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            if (u > 0 && q0 + u * (int)blockDim.x >= cnt) break;
-            L.x[kk[u] + (kColour == 0 ? 0 : 1)] = o0[u];
-            L.x[kk[u] + (kColour == 0 ? np + 1 : np)] = o1[u];
-        }
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+        const int k = 2 * q + 2 * patch_row(q, nc, L.rcp) * nc;
+        T o0, o1;
+        if (kColour == 0)
+            patch_red(L, L.x, L.b, k, o0, o1);
+        else
+            patch_black(L, L.x, L.b, k, o0, o1);
+        L.x[k + (kColour == 0 ? 0 : 1)] = o0;
+        L.x[k + (kColour == 0 ? np + 1 : np)] = o1;
     }
 }
 
 template <class T>
 __device__ __forceinline__ void pass_black_prolong(const PLvl<T>& L, const PLvl<T>& C) {
-    constexpr int kU = kPatchUnroll<T>;
     const int nc = L.nc, cnt = nc * nc, np = L.np, npc = C.np;
-    const unsigned rcp = L.rcp;
-    for (int q0 = threadIdx.x; q0 < cnt; q0 += kU * blockDim.x) {
-        T o0[kU], o1[kU];
-        int kk[kU];
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            const int q = q0 + u * blockDim.x;
-            if (u > 0 && q >= cnt) break;
-            const int I = patch_row(q, nc, rcp);
-            kk[u] = 2 * q + 2 * I * nc;
-            patch_black_prolong(L, L.x, L.b, kk[u], C.x, q + I * (npc - nc), npc, o0[u], o1[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < kU; ++u) {
-            if (u > 0 && q0 + u * (int)blockDim.x >= cnt) break;
-            L.x[kk[u] + 1] = o0[u];
-            L.x[kk[u] + np] = o1[u];
-        }
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+        const int I = patch_row(q, nc, L.rcp), k = 2 * q + 2 * I * nc;
+        T o0, o1;
+        patch_black_prolong(L, L.x, L.b, k, C.x, q + I * (npc - nc), npc, o0, o1);
+        L.x[k + 1] = o0;
+        L.x[k + np] = o1;
     }
 }
 
-template <class T>
+template <class T, bool kFromZero>
 __device__ __forceinline__ void pass_residual_restrict(const PLvl<T>& L, const PLvl<T>& C) {
     const int nc = L.nc, cnt = nc * nc, npc = C.np;
     for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
         const int I = patch_row(q, nc, L.rcp);
-        C.b[q + I * (npc - nc)] = patch_residual(L, L.x, L.b, 2 * q + 2 * I * nc);
+        C.b[q + I * (npc - nc)] = patch_residual<T, kFromZero>(L, L.x, L.b, 2 * q + 2 * I * nc);
     }
 }
 
@@ -324,7 +294,10 @@ __device__ void patch_cycle(const PLvl<T>* lv, int nlev, int pre, int post, int 
             pass_colour<T, 1>(A);
             __syncthreads();
         }
-        pass_residual_restrict(A, lv[lvl + 1]);
+        if (zero && pre == 1)
+            pass_residual_restrict<T, true>(A, lv[lvl + 1]);
+        else
+            pass_residual_restrict<T, false>(A, lv[lvl + 1]);
         __syncthreads();
     };
     auto ascend = [&](int lvl) {
@@ -424,8 +397,10 @@ __device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int 
                 red(A);
                 black(A);
             }
+            const bool from_zero = zero && pre == 1;
             for_patches_m(A, nrhs, [&](T* x, const T* b, int r, int k, int q, int I) {
-                C.b[r * stc + q + I * (npc - A.nc)] = patch_residual(A, x, b, k);
+                C.b[r * stc + q + I * (npc - A.nc)] =
+                    from_zero ? patch_residual<T, true>(A, x, b, k) : patch_residual<T, false>(A, x, b, k);
             });
             ++l;
             calls = (calls & ~(3ull << (2 * l))) | ((unsigned long long)gamma << (2 * l));
