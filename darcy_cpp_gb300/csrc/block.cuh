@@ -172,6 +172,7 @@ __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sb
             M.nc = (int)(np / 2);
             M.np = (int)np;
             M.rcp = row_reciprocal(M.nc);
+            M.rper = row_reciprocal(M.nc * M.nc);
             M.x = (T*)gtake(w * np, w * st * ntail, 0);
             M.b = (T*)gtake(w * np, w * st * ntail, 0);
             if (fp32) {
@@ -453,7 +454,8 @@ __device__ void block_build_tail(const BatchArgs& A, const BlockViews<T>& V) {
         L.b[j * st + k] = (k == j && j / L.np < L.n && j % L.np < L.n) ? T(1) : T(0);
     }
     __syncthreads();
-    patch_cycle_m<T>(V.lm, tl, V.nlev, A.pre, A.post, A.gamma, N, sizeof(T) == 4 ? V.h[V.nlev - 1].id : nullptr);
+    patch_cycle_m<T>(V.lm, tl, V.nlev, A.pre, A.post, A.gamma, A.gamma, N,
+                     sizeof(T) == 4 ? V.h[V.nlev - 1].id : nullptr);
     for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
         const int j = t / N, k = t - j * N;
         V.tail[k * pitch + j] = L.x[j * st + k];

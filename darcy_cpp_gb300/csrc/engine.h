@@ -120,9 +120,6 @@ template <class T>
 void launch_prolong_gs1(const Lvl<T>& L, const T* xc, CgState* st, cudaStream_t s);
 template <class T>
 void launch_gs0_dot(const Lvl<T>& L, const double* r, CgState* st, double* partials, cudaStream_t s);
-template <class T>
-void launch_tail(const Lvl<T>* lv_dev, int l0, int nlev, int pre, int post, int gamma, int top_calls,
-                 const double* id64, CgState* st, int threads, cudaStream_t s);
 // Dense coarse-tail operator: columns (setup) and application (per visit).
 void launch_tail_columns(const Lvl64* h_dev, const Lvl64* h_host, int l0, int nlev, int pre, int post, int gamma,
                          int top_calls, int N, double* Td, float* Tf, cudaStream_t s);

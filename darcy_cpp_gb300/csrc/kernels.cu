@@ -15,7 +15,6 @@
 #include <map>
 
 #include "block.cuh"
-#include "cycle.cuh"
 #include "engine.h"
 #include "fused.cuh"
 
@@ -626,51 +625,95 @@ __global__ void k_copy_back(const T* __restrict__ src, double* __restrict__ dst,
     for (int64_t k = GridScope::start(); k < m; k += GridScope::stride()) dst[k] = (double)src[k];
 }
 
-// Coarse tail: one CTA runs `top_calls` cycles on levels l0 .. nlev-1.
-template <class T>
-__global__ void k_tail(const Lvl<T>* __restrict__ lv, int l0, int nlev, int pre, int post, int gamma,
-                       int top_calls, const double* id64, const CgState* st) {
-    pdl_enter();
-    if (st && st->done) return;
-    block_cycle<T>(lv, l0, nlev, pre, post, gamma, top_calls, id64);
-}
-
 // Dense coarse tail. The levels from l0 down form a fixed linear map
 // b_{l0} -> x_{l0} ("x = 0, then top_calls cycles": multigrid.hpp:116-118 for
 // l0 > 0, multigrid.hpp:88-93 for l0 = 0). Column j is that map applied to the
-// unit vector e_j, computed by one CTA per column with the level vectors in
-// shared memory and the coefficients read from the (FP64) hierarchy. Stored
-// row-major, FP64 and optionally rounded to FP32 for the mixed form.
+// unit vector e_j, in FP64, stored row-major, FP64 and optionally rounded to
+// FP32 for the mixed form.
+//
+// A CTA computes `per` columns at once, the levels' coefficients (padded,
+// patch.cuh) and all its columns' vectors in shared memory: the ~150 dependent
+// passes are shared by 7 columns, and the side-2 level and what is below it is
+// one thread's work. A column at a time, cell by cell, spent its time in ~400
+// barriers and in integer divisions: 493 -> 252 us for 1024 columns of side 32
+// (of which the FP64 pipe needs ~105 us), 300 -> 163 us for 289 of side 17. The
+// arithmetic and its order are those of the level loops, so are the
+// operator's bits.
+//
 // k_tail_matvec reads T before its programmatic-launch wait, so this kernel
 // waits for its predecessor but does not release its dependents early: the
 // next kernel starts only once T is complete. (Under programmatic launch a
 // kernel's pre-wait code overlaps only its immediate predecessor, which
 // itself started after the kernel before it had completed; data written two
 // or more kernels earlier is safe to read before the wait.)
-__global__ void k_tail_columns(const Lvl64* __restrict__ h, int l0, int nlev, int pre, int post, int gamma,
-                               int top_calls, int N, double* __restrict__ Td, float* __restrict__ Tf) {
+constexpr int kTailColThreads = 512;
+
+// Shared-memory layout of the columns kernel: the levels from l0 down.
+// sbase == null: size only.
+__host__ __device__ inline size_t carve_tail(const int* sides, int l0, int nlev, int per, char* sbase,
+                                             PLvl<double>* lv) {
+    size_t off = 0;
+    auto take = [&](size_t lead, size_t count) -> double* {  // counts of doubles, 16-byte steps
+        lead = (lead + 1) & ~(size_t)1;
+        double* p = sbase ? (double*)sbase + off + lead : nullptr;
+        off += lead + ((count + 1) & ~(size_t)1);
+        return p;
+    };
+    for (int l = l0; l < nlev; ++l) {
+        const int n = sides[l], nc = (n + 1) / 2, np = 2 * nc;
+        const size_t m = (size_t)np * np, st = (size_t)rhs_stride(np);
+        PLvl<double> V{};
+        V.n = n;
+        V.nc = nc;
+        V.np = np;
+        V.rcp = row_reciprocal(nc);
+        V.rper = row_reciprocal(nc * nc);
+        V.e = take(2, m);
+        V.nf = take(np, m);
+        V.d = take(0, m);
+        V.id = take(0, m);
+        V.x = take(np, st * per);
+        V.b = take(np, st * per);
+        if (lv) lv[l] = V;
+    }
+    return off * sizeof(double);
+}
+
+struct TailSides {
+    int n[kMaxLevels];
+};
+
+__global__ void __launch_bounds__(kTailColThreads)
+    k_tail_columns(const Lvl64* __restrict__ h, TailSides sides, int l0, int nlev, int pre, int post, int gamma,
+                   int top_calls, int N, int per, double* __restrict__ Td, float* __restrict__ Tf) {
     pdl_wait();
-    extern __shared__ double sm_vec[];
-    __shared__ Lvl<double> lv[kMaxLevels];
-    if (threadIdx.x == 0) {
-        double* ptr = sm_vec;
-        for (int l = l0; l < nlev; ++l) {
-            const Lvl64 H = h[l];
-            const int m = H.n * H.n;
-            lv[l] = Lvl<double>{H.n, H.e, H.nf, H.d, H.id, ptr, ptr + m};
-            ptr += 2 * m;
+    extern __shared__ __align__(16) double sm_vec[];
+    __shared__ PLvl<double> lv[kMaxLevels];
+    const size_t bytes = carve_tail(sides.n, l0, nlev, per, (char*)sm_vec, threadIdx.x == 0 ? lv : nullptr);
+    for (size_t t = threadIdx.x; t < bytes / sizeof(double); t += blockDim.x) sm_vec[t] = 0.0;
+    __syncthreads();
+    for (int l = l0; l < nlev; ++l) {
+        const PLvl<double>& A = lv[l];
+        const Lvl64 H = h[l];
+        const int n = H.n;
+        for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
+            const int i = k / n, j = k - i * n, c = i * A.np + j;
+            ((double*)A.e)[c] = j + 1 < n ? H.e[k] : 0.0;
+            ((double*)A.nf)[c] = i + 1 < n ? H.nf[k] : 0.0;
+            ((double*)A.d)[c] = H.d[k];
+            ((double*)A.id)[c] = H.id[k];
         }
     }
+    const PLvl<double>& A = lv[l0];
+    const int j0 = blockIdx.x * per, cols = min(per, N - j0), n = A.n, st = rhs_stride(A.np);
+    for (int r = threadIdx.x; r < cols; r += blockDim.x) A.b[r * st + (j0 + r) / n * A.np + (j0 + r) % n] = 1.0;
     __syncthreads();
-    const int j = blockIdx.x;
-    double* b = lv[l0].b;
-    for (int k = threadIdx.x; k < N; k += blockDim.x) b[k] = (k == j) ? 1.0 : 0.0;
-    __syncthreads();
-    block_cycle<double>(lv, l0, nlev, pre, post, gamma, top_calls, nullptr);
-    const double* x = lv[l0].x;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        Td[(size_t)i * N + j] = x[i];
-        if (Tf) Tf[(size_t)i * N + j] = (float)x[i];
+    patch_cycle_m<double, true>(lv, l0, nlev, pre, post, gamma, top_calls, cols, nullptr);
+    for (int t = threadIdx.x; t < N * cols; t += blockDim.x) {
+        const int i = t / cols, r = t - i * cols;
+        const double v = A.x[r * st + i / n * A.np + i % n];
+        Td[(size_t)i * N + j0 + r] = v;
+        if (Tf) Tf[(size_t)i * N + j0 + r] = (float)v;
     }
 }
 
@@ -847,17 +890,16 @@ void launch_gs0_dot(const Lvl<T>& L, const double* r, CgState* st, double* parti
         launch_k(k_gs0_dot<T, false>, grid_fill(k_gs0_dot<T, false>, colour_count(L.n, 0)), kThreads, 0, s, L, r, st,
                  partials);
 }
-template <class T>
-void launch_tail(const Lvl<T>* lv_dev, int l0, int nlev, int pre, int post, int gamma, int top_calls,
-                 const double* id64, CgState* st, int threads, cudaStream_t s) {
-    launch_k(k_tail<T>, 1, threads, 0, s, lv_dev, l0, nlev, pre, post, gamma, top_calls, id64, st);
-}
 void launch_tail_columns(const Lvl64* h_dev, const Lvl64* h_host, int l0, int nlev, int pre, int post, int gamma,
                          int top_calls, int N, double* Td, float* Tf, cudaStream_t s) {
-    size_t smem = 0;
-    for (int l = l0; l < nlev; ++l) smem += 2 * sizeof(double) * (size_t)h_host[l].n * h_host[l].n;
+    TailSides sides{};
+    for (int l = 0; l < nlev; ++l) sides.n[l] = h_host[l].n;
+    // one wave of one CTA an SM: 7 columns each for the 1024 columns of side 32
+    const int per = std::min(8, (N + 151) / 152);
+    const size_t smem = carve_tail(sides.n, l0, nlev, per, nullptr, nullptr);
     cudaFuncSetAttribute(k_tail_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_k(k_tail_columns, N, 256, smem, s, h_dev, l0, nlev, pre, post, gamma, top_calls, N, Td, Tf);
+    launch_k(k_tail_columns, (N + per - 1) / per, kTailColThreads, smem, s, h_dev, sides, l0, nlev, pre, post, gamma,
+             top_calls, N, per, Td, Tf);
 }
 template <class T>
 void launch_tail_matvec(const T* M, int N, const T* b, T* x, CgState* st, cudaStream_t s) {
@@ -1200,8 +1242,6 @@ void launch_block_solve(const BatchArgs& args, int ctas, int threads, cudaStream
     template void launch_residual_restrict<T>(const Lvl<T>&, T*, CgState*, cudaStream_t);                  \
     template void launch_prolong_gs1<T>(const Lvl<T>&, const T*, CgState*, cudaStream_t);                  \
     template void launch_gs0_dot<T>(const Lvl<T>&, const double*, CgState*, double*, cudaStream_t);        \
-    template void launch_tail<T>(const Lvl<T>*, int, int, int, int, int, int, const double*, CgState*, int, \
-                                 cudaStream_t);                                                            \
     template void launch_dot_rz<T>(const T*, const double*, int64_t, CgState*, double*, cudaStream_t);     \
     template void launch_tail_matvec<T>(const T*, int, const T*, T*, CgState*, cudaStream_t);              \
     template void launch_visit_pre<T>(const VisitLevel<T>&, const T*, T*, T*, cudaStream_t);                 \

@@ -25,7 +25,8 @@ namespace dgpu {
 template <class T>
 struct PLvl {
     int n, nc, np;
-    unsigned rcp;  // ceil(2^32 / nc) while the product below is exact, else 0
+    unsigned rcp;   // ceil(2^32 / nc) while the product below is exact, else 0
+    unsigned rper;  // the same for nc^2 (levels with many right-hand sides)
     const T* e;
     const T* nf;
     const T* d;
@@ -168,6 +169,70 @@ __device__ __forceinline__ T patch_residual(const PLvl<T>& L, const T* x, const 
     v0 += L.nf[k - np] * x[k - np];
     v1 += n0.y * x01;
     return v0 + v1;
+}
+
+// The same sum over all four cells, each residual rounded on its own, cells in
+// row-major order and products in the order of cell_residual (the first two
+// terms as e x_E subtracted from the rounded d x): the grid engine's rounding,
+// which its tail operator keeps.
+__device__ __forceinline__ double patch_residual_all(const PLvl<double>& L, const double* x, const double* b, int k) {
+    const int np = L.np;
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int q = k + (c >> 1) * np + (c & 1);
+        double v = fma(-L.e[q], x[q + 1], __dmul_rn(L.d[q], x[q]));
+        v = fma(-L.e[q - 1], x[q - 1], v);
+        v = fma(-L.nf[q], x[q + np], v);
+        v = fma(-L.nf[q - np], x[q - np], v);
+        s += b[q] - v;
+    }
+    return s;
+}
+
+// `calls` calls from zero of the side-2 level A, and of the 1 x 1 level below
+// it (reciprocal diagonal idc), for one right-hand side, by one thread: the
+// level has one patch, and its ~10 passes in one step save the CTA as many
+// barrier-separated ones. Arithmetic and order as the passes with
+// patch_residual_all; terms of absent neighbours (zero faces) left out.
+__device__ __forceinline__ void solve_side2(const PLvl<double>& A, double idc, const double* b, double* x, int pre,
+                                            int post, int calls) {
+    const double e0 = A.e[0], e1 = A.e[2], n0 = A.nf[0], n1 = A.nf[1];
+    const double b0 = b[0], b1 = b[1], b2 = b[2], b3 = b[3];
+    const double i0 = A.id[0], i1 = A.id[1], i2 = A.id[2], i3 = A.id[3];
+    // (products and sums that must round on their own are kept from contracting)
+    double x0 = __dmul_rn(b0, i0), x1 = 0.0, x2 = 0.0, x3 = __dmul_rn(b3, i3);  // colour 0 from a zero iterate
+    // cells 0, 3: colour 0; cells 1, 2: colour 1; terms east, west, north, south
+    auto red = [&] {
+        x0 = __dmul_rn(fma(n0, x2, fma(e0, x1, b0)), i0);
+        x3 = __dmul_rn(fma(n1, x1, fma(e1, x2, b3)), i3);
+    };
+    auto black = [&](double c0, double c3) {
+        x1 = __dmul_rn(fma(n1, c3, fma(e0, c0, b1)), i1);
+        x2 = __dmul_rn(fma(n0, c0, fma(e1, c3, b2)), i2);
+    };
+    for (int call = 0; call < calls; ++call) {
+        black(x0, x3);
+        for (int s = 1; s < pre; ++s) {
+            red();
+            black(x0, x3);
+        }
+        double s = b0 - fma(-n0, x2, fma(-e0, x1, __dmul_rn(A.d[0], x0)));
+        s += b1 - fma(-n1, x3, fma(-e0, x0, __dmul_rn(A.d[1], x1)));
+        s += b2 - fma(-n0, x0, fma(-e1, x3, __dmul_rn(A.d[2], x2)));
+        s += b3 - fma(-n1, x1, fma(-e1, x2, __dmul_rn(A.d[3], x3)));
+        const double c = __dmul_rn(s, idc);  // the 1 x 1 level, exactly; prolonged to the patch
+        black(__dadd_rn(x0, c), __dadd_rn(x3, c));
+        for (int q = 1; q < post; ++q) {
+            red();
+            black(x0, x3);
+        }
+        red();
+    }
+    x[0] = x0;
+    x[1] = x1;
+    x[2] = x2;
+    x[3] = x3;
 }
 
 // ------------------------------------------------------------ CTA passes
@@ -346,9 +411,11 @@ __device__ void patch_cycle(const PLvl<T>* lv, int nlev, int pre, int post, int 
 
 // -------------------------------------------------- many right-hand sides
 //
-// The recursion below level `l0` for `nrhs` right-hand sides at once (gamma
-// calls from zero at l0), used to build the dense tail. Right-hand side r of
-// a level is at x + r * stride, b + r * stride, stride = np^2 + 2 np.
+// `top` calls of level l0 from zero for `nrhs` right-hand sides at once, used
+// to build a dense operator of the levels from l0 down. Right-hand side r of a
+// level is at x + r * stride, b + r * stride, stride = np^2 + 2 np. id64: the
+// FP64 reciprocal diagonal of the 1 x 1 level (FP32 cycle), or null. kAll (FP64):
+// residuals by patch_residual_all, the side-2 level by solve_side2.
 
 __host__ __device__ inline int rhs_stride(int np) { return np * np + 2 * np; }
 
@@ -356,17 +423,18 @@ template <class T, class F>
 __device__ __forceinline__ void for_patches_m(const PLvl<T>& L, int nrhs, F&& f) {
     const int nc = L.nc, per = nc * nc, st = rhs_stride(L.np);
     for (int t = threadIdx.x; t < per * nrhs; t += blockDim.x) {
-        const int r = t / per, q = t - r * per;
+        const int r = patch_row(t, per, L.rper), q = t - r * per;
         const int I = patch_row(q, nc, L.rcp);
         f(L.x + r * st, L.b + r * st, r, 2 * q + 2 * I * nc, q, I);
     }
     __syncthreads();
 }
 
-template <class T>
-__device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int post, int gamma, int nrhs,
+template <class T, bool kAll = false>
+__device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int post, int gamma, int top, int nrhs,
                               const double* id64) {
-    unsigned long long calls = (unsigned long long)gamma << (2 * l0);
+    const int lb = kAll && nlev >= 2 && nlev - 2 >= l0 ? nlev - 2 : nlev - 1;  // the side-2 or the 1 x 1 level
+    unsigned long long calls = (unsigned long long)top << (2 * l0);
     int l = l0;
     bool zero = true;
     auto red = [&](const PLvl<T>& A) {
@@ -386,7 +454,7 @@ __device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int 
         });
     };
     for (;;) {
-        while (l + 1 < nlev) {
+        while (l < lb) {
             const PLvl<T>& A = lv[l];
             const PLvl<T>& C = lv[l + 1];
             const int stc = rhs_stride(C.np), npc = C.np;
@@ -399,24 +467,36 @@ __device__ void patch_cycle_m(const PLvl<T>* lv, int l0, int nlev, int pre, int 
             }
             const bool from_zero = zero && pre == 1;
             for_patches_m(A, nrhs, [&](T* x, const T* b, int r, int k, int q, int I) {
-                C.b[r * stc + q + I * (npc - A.nc)] =
-                    from_zero ? patch_residual<T, true>(A, x, b, k) : patch_residual<T, false>(A, x, b, k);
+                T s;
+                if constexpr (kAll)
+                    s = patch_residual_all(A, x, b, k);
+                else
+                    s = from_zero ? patch_residual<T, true>(A, x, b, k) : patch_residual<T, false>(A, x, b, k);
+                C.b[r * stc + q + I * (npc - A.nc)] = s;
             });
             ++l;
             calls = (calls & ~(3ull << (2 * l))) | ((unsigned long long)gamma << (2 * l));
             zero = true;
         }
-        {  // the 1 x 1 level
+        {  // the bottom: level lb and what is below it
             const PLvl<T>& A = lv[l];
             const int st = rhs_stride(A.np);
-            for (int r = threadIdx.x; r < nrhs; r += blockDim.x)
+            for (int r = threadIdx.x; r < nrhs; r += blockDim.x) {
+                if constexpr (kAll) {
+                    if (A.n == 2) {
+                        solve_side2(A, lv[l + 1].id[0], A.b + r * st, A.x + r * st, pre, post,
+                                    (int)((calls >> (2 * l)) & 3ull));
+                        continue;
+                    }
+                }
                 A.x[r * st] = id64 ? (T)((double)A.b[r * st] * id64[0]) : A.b[r * st] * A.id[0];
+            }
             __syncthreads();
-            calls &= ~(3ull << (2 * l));  // further calls of it change nothing
+            calls &= ~(3ull << (2 * l));  // done (further calls of the 1 x 1 level change nothing)
         }
         for (;;) {
             if (((calls >> (2 * l)) & 3ull) != 0) calls -= 1ull << (2 * l);
-            if (l + 1 < nlev && ((calls >> (2 * l)) & 3ull) != 0) break;
+            if (l < lb && ((calls >> (2 * l)) & 3ull) != 0) break;
             if (l == l0) return;
             --l;
             const PLvl<T>& A = lv[l];
