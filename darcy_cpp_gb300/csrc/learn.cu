@@ -72,6 +72,8 @@ typedef __nv_bfloat16 bf16;
 struct Geom {
     int H, W, P, tiles_per_img, nq;  // nq: staged positions per tile (multiple of 8)
     int step_r, step_c;              // kTile positions = step_r rows + step_c columns of pitch P
+    int step32_r, step32_c;          // 32 positions
+    unsigned rp;                     // ceil(2^32 / P): s / P as a high product, exact for s P < 2^32
 };
 
 inline bool side_supported(int s) { return s >= 8 && s <= kMaxSide && (s % 2) == 0; }
@@ -84,6 +86,9 @@ inline Geom make_geom(int side) {
     g.nq = ((kTile + 2 * g.P + 2) + 7) & ~7;
     g.step_r = kTile / g.P;
     g.step_c = kTile % g.P;
+    g.step32_r = 32 / g.P;
+    g.step32_c = 32 % g.P;
+    g.rp = (unsigned)((0x100000000ull + g.P - 1) / g.P);
     return g;
 }
 
@@ -94,10 +99,33 @@ __device__ __forceinline__ void tile_origin(int64_t t, const Geom& g, int64_t& p
     pbase = b * (int64_t)g.H * g.W;
 }
 
+// The tiles blockIdx.x, blockIdx.x + gridDim.x, ... in turn: first pixel of the
+// tile's image and first padded position, one division at the start.
+struct TileWalk {
+    int64_t pixel;
+    int s0, in_img, step_img, step_tile;
+    __device__ __forceinline__ explicit TileWalk(const Geom& g) {
+        tile_origin(blockIdx.x, g, pixel, s0);
+        in_img = s0 / kTile;
+        step_img = (int)(gridDim.x / (unsigned)g.tiles_per_img);
+        step_tile = (int)(gridDim.x - (unsigned)step_img * g.tiles_per_img);
+    }
+    __device__ __forceinline__ void step(const Geom& g) {
+        in_img += step_tile;
+        int images = step_img;
+        if (in_img >= g.tiles_per_img) {
+            in_img -= g.tiles_per_img;
+            images += 1;
+        }
+        pixel += (int64_t)images * (g.H * g.W);
+        s0 = in_img * kTile;
+    }
+};
+
 // Pixel index (within the image) of padded position s, or -1 outside it.
 __device__ __forceinline__ int position_pixel(const Geom& g, int s) {
     if (s < 0) return -1;
-    const int r = s / g.P, c = s - r * g.P;
+    const int r = (int)__umulhi((unsigned)s, g.rp), c = s - r * g.P;
     if (r >= g.H || c < 1 || c > g.W) return -1;
     return r * g.W + c - 1;
 }
@@ -110,7 +138,7 @@ struct PosRC {
 };
 __device__ __forceinline__ PosRC position_rc(const Geom& g, int s) {
     const int t = s + 2 * g.P;
-    const int r = t / g.P;
+    const int r = (int)__umulhi((unsigned)t, g.rp);
     return PosRC{r - 2, t - r * g.P};
 }
 __device__ __forceinline__ PosRC rc_add(const Geom& g, PosRC p, int dr, int dc) {
@@ -272,15 +300,18 @@ __device__ __forceinline__ float apply_a(const float* __restrict__ v, const floa
     return y;
 }
 
-constexpr int kEnergyThreads = 256;
+constexpr int kEnergyThreads = 1024;  // one CTA a sample: 256 threads left each with a long chain of stencils
+                                      // (batch of 256, 64 x 64: 30 -> 17 us)
 
 __device__ __forceinline__ double block_sum_d(double v, double* red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+    if (threadIdx.x < 32) {
+        t = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    }
     __syncthreads();
     return t;  // valid in thread 0
 }
@@ -325,13 +356,15 @@ __global__ void __launch_bounds__(kEnergyThreads) k_energy_loss(const float* __r
     if (threadIdx.x == 0) part[blockIdx.x] = (float)(tot / (double)norm[blockIdx.x]);
 }
 
-// loss = mean of the per-sample parts, summed in order.
-__global__ void k_mean_parts(const float* __restrict__ part, int n, float* __restrict__ loss) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int q = 0; q < n; ++q) s += part[q];
-        *loss = (float)(s / (double)n);
-    }
+// loss = mean of the per-sample parts, summed in a fixed order (a chain of
+// FP64 adds in one thread, ~70 ns each, took 21 us for 256 samples).
+__global__ void __launch_bounds__(kEnergyThreads) k_mean_parts(const float* __restrict__ part, int n,
+                                                               float* __restrict__ loss) {
+    __shared__ double red[kEnergyThreads / 32];
+    double s = 0.0;
+    for (int q = threadIdx.x; q < n; q += kEnergyThreads) s += part[q];
+    const double tot = block_sum_d(s, red);
+    if (threadIdx.x == 0) *loss = (float)(tot / (double)n);
 }
 
 // u0 = out * uscale * f / fref in FP64.
@@ -444,11 +477,63 @@ __global__ void k_conv_simt(const TIN* __restrict__ x, const bf16* __restrict__ 
     }
 }
 
+// The output layer's input gradient: a 1 -> 32 channel convolution of the FP32
+// dout with the flipped weights wB[co][tap], times GELU'(aux). One thread per
+// (pixel, 8 channels): the nine neighbours are read once for eight outputs and
+// the pre-activations and results move as 16-byte vectors; every output's sum
+// has k_conv_simt's order. Bound by the erf and exp of GELU' (~50 instructions
+// an output): 383 us with one thread an output and its 64-bit divisions, 72
+// us now (256 fields of 64 x 64).
+__global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dout, const bf16* __restrict__ wB, int H,
+                                                   int W, int64_t npix, const float* __restrict__ aux,
+                                                   bf16* __restrict__ act) {
+    __shared__ float sw[kTaps][kC];
+    for (int q = threadIdx.x; q < kTaps * kC; q += blockDim.x)
+        sw[q % kTaps][q / kTaps] = __bfloat162float(wB[q]);
+    __syncthreads();
+    const int hw = H * W, part = threadIdx.x & 3;  // channels 8 part .. 8 part + 7
+    for (int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 2; p < npix;
+         p += ((int64_t)gridDim.x * blockDim.x) >> 2) {
+        const int64_t img = p < (1ll << 31) ? (int64_t)((unsigned)p / (unsigned)hw) : p / hw;
+        const int rem = (int)(p - img * hw), i = rem / W, j = rem - i * W;
+        float acc[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+#pragma unroll
+        for (int tap = 0; tap < kTaps; ++tap) {
+            const int di = tap / 3 - 1, dj = tap % 3 - 1;
+            const bool in = i + di >= 0 && i + di < H && j + dj >= 0 && j + dj < W;
+            const float v = in ? dout[p + di * W + dj] : 0.f;
+            if (in)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) acc[c] += v * sw[tap][part * 8 + c];
+        }
+        const float4* z = reinterpret_cast<const float4*>(aux + p * kC + part * 8);
+        const float4 z0 = z[0], z1 = z[1];
+        const float g[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(acc[2 * e] * gelu_grad(g[2 * e]),
+                                                            acc[2 * e + 1] * gelu_grad(g[2 * e + 1]));
+            o[e] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        *reinterpret_cast<uint4*>(act + p * kC + part * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
 // ------------------------------------------------- tensor-core convolution
 //
 // One 3x3 layer as an implicit GEMM, 128 threads (4 warps) per CTA, one tile
-// of 128 padded positions at a time, the next tile's input staged (cp.async)
-// while the current one is multiplied and written back.
+// of 128 padded positions at a time, as a pipeline of three: while tile i is
+// written back from one accumulator, tile i + 1 is multiplied into the other
+// and tile i + 2 is staged (cp.async). Bound by the epilogue's arithmetic (the
+// erf of GELU: most of ~1300 instructions a warp and tile; the ALU pipe is
+// 53-60% busy). A 32 -> 32 layer of 1024 fields of 64 x 64: 312 us when a tile
+// was multiplied and written back one after the other, its staging read every
+// sector twice and descriptors were rebuilt for each multiplication; 257 us now.
+// (Two such groups sharing the weights, one staging buffer each, 32 warps an
+// SM instead of 16: more instructions, 279 us.)
 //
 // Template: CCH = 16-byte input chunks per pixel (4: 32 channels; 1: the
 // 8-channel padded input of the first layer); NOUT = GEMM N (32 channels, or
@@ -466,13 +551,15 @@ __global__ void k_conv_simt(const TIN* __restrict__ x, const bf16* __restrict__ 
 // Epilogues: kEpiGelu (pre-activation FP32 if `pre`, GELU -> BF16 act),
 // kEpiGeluGrad (act = acc * GELU'(aux), BF16), kEpiLinear (outf = acc[0] + b).
 constexpr int kConvThreads = 128;
+constexpr int kConvCols = 64;  // tensor-memory columns: two accumulators of 32
 constexpr long long kWaitLimit = 1ll << 24;  // mbarrier polls before a wait is declared lost
 
 template <int CCH, int NOUT>
 struct TcShape {
     static constexpr int KCH = CCH == 4 ? 36 : 10;            // K chunks of B
     static constexpr int SLICES = CCH == 4 ? 18 : 5;
-    static constexpr int B_BYTES = KCH * NOUT * 16;
+    static constexpr int B_CHUNK = NOUT * 16;                 // bytes from one K chunk of B to the next
+    static constexpr int B_BYTES = KCH * B_CHUNK;
     static constexpr int K = KCH * 8;                         // bf16 per weight row
 };
 
@@ -488,16 +575,23 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool v
                  : "memory");
 }
 
+// Lanes take the chunks of a pixel first (four lanes 64 contiguous bytes, a
+// warp 512): with the lanes along the pixels and one chunk an instruction,
+// every 32-byte sector was fetched twice and a warp's copy touched 16 lines.
+// The positions a thread steps through are 128 / CCH apart.
 template <int CCH>
 __device__ __forceinline__ void stage_tile(const bf16* __restrict__ x, const Geom& g, int64_t pbase, int s0,
                                            uint32_t buf, uint32_t plane) {
-    PosRC pos = position_rc(g, s0 - g.P - 1 + (int)threadIdx.x);
-    for (int q = threadIdx.x; q < g.nq; q += kConvThreads) {
+    constexpr int kStep = kConvThreads / CCH;
+    const int chunk = threadIdx.x % CCH, q0 = threadIdx.x / CCH;
+    const int dr = kStep == kTile ? g.step_r : g.step32_r, dc = kStep == kTile ? g.step_c : g.step32_c;
+    const bf16* xi = x + pbase * (CCH * 8) + chunk * 8;
+    const uint32_t dst = buf + chunk * plane;
+    PosRC pos = position_rc(g, s0 - g.P - 1 + q0);
+    for (int q = q0; q < g.nq; q += kStep) {
         const int pix = rc_pixel(g, pos);
-        const bf16* src = pix >= 0 ? x + (pbase + pix) * CCH * 8 : x;
-#pragma unroll
-        for (int c = 0; c < CCH; ++c) cp_async16(buf + c * plane + q * 16, src + c * 8, pix >= 0);
-        pos = rc_add(g, pos, g.step_r, g.step_c);
+        cp_async16(dst + q * 16, pix >= 0 ? xi + pix * (CCH * 8) : x, pix >= 0);
+        pos = rc_add(g, pos, dr, dc);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
@@ -514,106 +608,111 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict
     const uint32_t stage = tc_stage_bytes(CCH, g.nq);
     unsigned char* sB = sm;
     float* sBias = reinterpret_cast<float*>(sm + S::B_BYTES + 2 * stage);
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + S::B_BYTES + 2 * stage + 128);
+    uint64_t* mbar_at = reinterpret_cast<uint64_t*>(sm + S::B_BYTES + 2 * stage + 128);
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t plane = g.nq * 16;
 
     for (int q = tid; q < NOUT * S::KCH; q += kConvThreads) {
         const int n = q / S::KCH, c = q - n * S::KCH;
-        *reinterpret_cast<uint4*>(sB + c * (NOUT * 16) + n * 16) =
+        *reinterpret_cast<uint4*>(sB + c * S::B_CHUNK + n * 16) =
             *reinterpret_cast<const uint4*>(wB + (size_t)n * S::K + c * 8);
     }
     if (tid < 32) sBias[tid] = (bias && tid < NOUT) ? bias[tid] : 0.f;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(32u)
+                     "r"((uint32_t)kConvCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) mbar_init(smem_u32(mbar), 1);
+    if (tid == 0) mbar_init(smem_u32(mbar_at), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem = tmem_base, mbar = smem_u32(mbar_at);
     const uint32_t b_addr = smem_u32(sB), x_addr = smem_u32(sm + S::B_BYTES);
     constexpr uint32_t idesc = mma_idesc(kTile, NOUT);
-    uint32_t phase = 0;
-    int buf = 0;
     // polls of this CTA's first completion wait (kWaitLimit unless a test
     // shortens it to make the wait run out); every later wait, and the drain
     // wait after one ran out, keeps kWaitLimit
     long long wait_polls = first_wait;
-
-    int64_t tile = blockIdx.x;
-    if (tile < ntiles) {
-        int64_t pb;
-        int s0;
-        tile_origin(tile, g, pb, s0);
-        stage_tile<CCH>(x, g, pb, s0, x_addr, plane);
-    }
-    for (; tile < ntiles; tile += gridDim.x) {
-        int64_t pbase;
-        int s0;
-        tile_origin(tile, g, pbase, s0);
+    const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // this CTA's tiles, >= 1
+    TileWalk ahead(g), here(g);  // the tile to stage next, the tile to write back
+    auto stage_next = [&](int i) {
+        if (i < mine) {
+            stage_tile<CCH>(x, g, ahead.pixel, ahead.s0, x_addr + (i & 1) * stage, plane);
+            ahead.step(g);
+        }
+    };
+    auto multiply = [&](int i) {  // one thread
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // (a start address is the low 14 bits of its descriptor, in 16-byte
+        // units: the slices differ by small sums added to one descriptor)
+        const uint32_t xb = x_addr + (i & 1) * stage, acc = tmem + (i & 1) * 32;
+        const uint64_t b0 = smem_desc(b_addr, S::B_CHUNK, 128);
+        if constexpr (CCH == 4) {
+            const uint64_t a0 = smem_desc(xb, plane, 128);
+            const uint32_t half = 2 * (plane >> 4);
+#pragma unroll
+            for (int sl = 0; sl < S::SLICES; ++sl) {
+                const int tap = sl >> 1, dy = tap / 3, dx = tap % 3;
+                mma_bf16(acc, a0 + (dy * (uint32_t)g.P + dx + (sl & 1) * half), b0 + sl * 2 * (S::B_CHUNK >> 4), idesc,
+                         sl > 0 ? 1u : 0u);
+            }
+        } else {
+#pragma unroll
+            for (int sl = 0; sl < S::SLICES; ++sl) {
+                const int t1 = 2 * sl, t2 = 2 * sl + 1 < 8 ? 2 * sl + 1 : 8;
+                const int sh1 = (t1 / 3) * g.P + t1 % 3, sh2 = (t2 / 3) * g.P + t2 % 3;
+                mma_bf16(acc, smem_desc(xb + sh1 * 16, (sh2 - sh1) * 16, 128), b0 + sl * 2 * (S::B_CHUNK >> 4), idesc,
+                         sl > 0 ? 1u : 0u);
+            }
+        }
+        mma_commit(mbar);
+    };
+    stage_next(0);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (tid == 0) multiply(0);
+    __syncwarp();
+    stage_next(1);
+    for (int i = 0; i < mine; ++i) {
+        // tile i + 1 has landed, tile i is multiplied, every thread has read
+        // the accumulator of tile i - 1
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        const uint32_t xb = x_addr + buf * stage;
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-            for (int sl = 0; sl < S::SLICES; ++sl) {
-                uint32_t a_start, lbo;
-                if (CCH == 4) {
-                    const int tap = sl >> 1, h = sl & 1;
-                    const int dy = tap / 3, dx = tap - dy * 3;
-                    a_start = xb + (2 * h) * plane + (dy * g.P + dx) * 16;
-                    lbo = plane;
-                } else {
-                    const int t1 = 2 * sl, t2 = min(2 * sl + 1, 8);
-                    const int sh1 = (t1 / 3) * g.P + t1 % 3, sh2 = (t2 / 3) * g.P + t2 % 3;
-                    a_start = xb + sh1 * 16;
-                    lbo = (sh2 - sh1) * 16;
-                }
-                mma_bf16(tmem, smem_desc(a_start, lbo, 128),
-                         smem_desc(b_addr + sl * 2 * (NOUT * 16), NOUT * 16, 128), idesc, sl > 0 ? 1u : 0u);
-            }
-            mma_commit(smem_u32(mbar));
-        }
-        // stage the next tile into the other buffer while this one is multiplied
-        const int64_t next = tile + gridDim.x;
-        if (next < ntiles) {
-            int64_t pb;
-            int s1;
-            tile_origin(next, g, pb, s1);
-            stage_tile<CCH>(x, g, pb, s1, x_addr + (buf ^ 1) * stage, plane);
-        }
-        __syncwarp();
-        const bool ok = __syncthreads_and(mbar_wait(smem_u32(mbar), phase, wait_polls));
+        const bool ok = __syncthreads_and(mbar_wait(mbar, (uint32_t)i & 1u, wait_polls));
         wait_polls = kWaitLimit;
-        phase ^= 1u;
         if (!ok) {
             if (tid == 0) atomicExch(err, 1);
             // give an MMA still in flight a bounded chance to land before the
             // tensor memory is released
-            mbar_wait(smem_u32(mbar), phase ^ 1u, kWaitLimit);
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            mbar_wait(mbar, (uint32_t)i & 1u, kWaitLimit);
             break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0 && i + 1 < mine) multiply(i + 1);
+        __syncwarp();
+        stage_next(i + 2);  // into the buffer tile i was multiplied from
         float v[32];
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
-        const int pix = position_pixel(g, s0 + tid);  // row tid of the tile
+        tmem_ld32(tmem + (i & 1) * 32 + ((uint32_t)(warp * 32) << 16), v);
+        const int pix = position_pixel(g, here.s0 + tid);  // row tid of the tile
         if (pix >= 0) {
-            const int64_t p = pbase + pix;
+            const int64_t p = here.pixel + pix;
             if (mode == kEpiLinear) {
                 outf[p] = v[0] + sBias[0];
             } else {
                 if (mode == kEpiGelu) {
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] += sBias[c];
+                    for (int c = 0; c < 32; c += 4) {
+                        const float4 bb = *reinterpret_cast<const float4*>(sBias + c);
+                        v[c] += bb.x;
+                        v[c + 1] += bb.y;
+                        v[c + 2] += bb.z;
+                        v[c + 3] += bb.w;
+                    }
                     if (pre) {
                         float4* dst = reinterpret_cast<float4*>(pre + p * kC);
 #pragma unroll
@@ -646,16 +745,16 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict
                 }
             }
         }
+        here.step(g);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();  // the accumulator and this buffer are reused two tiles on
-        buf ^= 1;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kConvCols)
+                     : "memory");
 }
 
 // ------------------------------------------------------- weight gradients
@@ -747,48 +846,72 @@ inline size_t wgrad_smem(const Geom& g, int cin, int cout) {
 }
 
 // Sums the per-CTA partials in CTA order into the layer's weight and bias
-// gradients (master layout: w[co][k], then b[co]).
-__global__ void k_reduce_wgrad(const float* __restrict__ part, int nparts, int nv, int K, float* __restrict__ gw,
-                               float* __restrict__ gb) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nv; j += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int q = 0; q < nparts; ++q) s += part[(int64_t)q * nv + j];
-        const int co = j / (K + 1), k = j - co * (K + 1);
-        if (k < K)
-            gw[co * K + k] = s;
-        else
-            gb[co] = s;
+// gradients (master layout: w[co][k], then b[co]): 32 values a block, loaded
+// by eight warps into shared memory, kReduceRows partials at a time, then
+// added in order by one warp. Bound by latency (one thread a value and its
+// chain of loads took 12.6 us for 152 x 9248 partials, 5.9 us now).
+constexpr int kReduceRows = 160;
+__global__ void __launch_bounds__(256) k_reduce_wgrad(const float* __restrict__ part, int nparts, int nv, int K,
+                                                      float* __restrict__ gw, float* __restrict__ gb) {
+    __shared__ float rows[kReduceRows][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
+    float s = 0.f;
+    for (int at = 0; at < nparts; at += kReduceRows) {
+        const int c = min(kReduceRows, nparts - at);
+        if (j < nv)
+#pragma unroll 10
+            for (int q = w; q < c; q += 8) rows[q][lane] = part[(int64_t)(at + q) * nv + j];
+        __syncthreads();
+        if (w == 0)
+#pragma unroll 8
+            for (int q = 0; q < c; ++q) s += rows[q][lane];
+        __syncthreads();
     }
+    if (w != 0 || j >= nv) return;
+    const int co = j / (K + 1), k = j - co * (K + 1);
+    if (k < K)
+        gw[co * K + k] = s;
+    else
+        gb[co] = s;
 }
 
 // Weight gradients on the tensor cores. The same sums as k_wgrad,
 // gW[co][tap * CIN + ci] = sum_p dy[p, co] x[p + shift(tap), ci] and
-// gb[co] = sum_p dy[p, co], as D = A B with M = (tap, input-channel chunk, ci)
-// rows, N = co columns and K = pixels: per tile of 128 positions the CTA
-// stages A as one 128-position plane per (tap, chunk of 8 input channels) --
-// each plane the staged input shifted by the tap (an im2col in shared memory,
-// 16-byte cp.async chunks) -- plus one plane of ones whose D row is the bias
-// gradient, zero planes up to a multiple of 16, and B as one plane per chunk
-// of 8 output channels. Both operands are MN-major core matrices (8 positions
-// x 16 bytes of channels, 128 contiguous bytes): A's 16-plane groups are the
-// M = 128 tiles, K advances 16 positions per MMA. One thread issues MT x 8
-// tcgen05.mma (M 128, N NOUT, K 16, BF16 in, FP32 accumulate) per tile into
-// MT tensor-memory accumulators that persist over all the CTA's tiles (the
-// next tile is staged while they run); at the end each warp reads its 32
-// rows with tcgen05.ld and writes the CTA's partial in the layout
-// k_reduce_wgrad sums in CTA order, so training stays deterministic.
+// gb[co] = sum_p dy[p, co], as D = A B with N = co columns and K = pixels. Per
+// tile of 128 positions the CTA stages the input as three bands, one per tap
+// row dy, of 130 positions each, in one plane per chunk of 8 input channels
+// (16-byte cp.async copies); in a plane, 8 positions x 16 bytes of channels
+// are an MN-major core matrix (128 contiguous bytes), so the 3 CCH planes, a
+// plane of ones (whose D row is the bias gradient) and zero planes up to 16
+// are the 128 rows (band, input channel) of A, uniformly strided, and the tap
+// column dx is a start 16 dx bytes into the planes: three accumulators, one
+// per dx, instead of nine shifted copies of the input. B is one plane per
+// chunk of 8 output channels. One thread issues 3 x 8 tcgen05.mma (M 128,
+// N NOUT, K 16, BF16 in, FP32 accumulate) per tile into tensor-memory
+// accumulators that persist over all the CTA's tiles (the next tile is staged
+// while they run); at the end each warp reads its 32 rows with tcgen05.ld and
+// writes the CTA's partial in the layout k_reduce_wgrad sums in CTA order, so
+// training stays deterministic.
 // An FP32 dy (the output layer's, one channel) enters as a BF16 hi/lo pair in
 // columns 0 and 1, summed in the epilogue.
+//
+// Bound by staging and its waits. With nine shifted copies (36 planes of 128
+// positions, 104 KB a stage, two stages) the kernel took 218 us on 256 fields
+// of 64 x 64; with the bands a stage is 43 KB, four of them are in flight, and
+// it takes 103 us. One CTA an SM, as before: the tiles of one accumulator and
+// their order, and so every gradient's bits, stay what they were.
 template <int CCH, int NOUT>
 struct WgradTc {
-    static constexpr int kDataPlanes = kTaps * CCH;                     // A planes holding x
-    static constexpr int MT = (kDataPlanes + 1 + 15) / 16;              // M = 128 tiles (with the ones plane)
-    static constexpr int kAPlanes = MT * 16;
+    static constexpr int kDataPlanes = 3 * CCH;                         // A planes holding x: plane dy * CCH + chunk
+    static constexpr int kAPlanes = 16;                                 // with the ones plane and zeros: M = 128
     static constexpr int kBPlanes = NOUT / 8;
-    static constexpr int kPlane = kTile * 16;                           // bytes: 128 positions x 16 B
-    static constexpr int kStage = (kAPlanes + kBPlanes) * kPlane;
-    static constexpr int kCols = MT * NOUT <= 32 ? 32 : MT * NOUT <= 64 ? 64 : MT * NOUT <= 128 ? 128 : 256;
-    static constexpr int kSmem = 2 * kStage + 16;
+    static constexpr int kPos = kTile + 4;                              // positions of an A plane (130 used)
+    static constexpr int kAPlane = kPos * 16;                           // bytes
+    static constexpr int kBPlane = kTile * 16;
+    static constexpr int kStage = kAPlanes * kAPlane + kBPlanes * kBPlane;
+    static constexpr int kCols = 3 * NOUT <= 64 ? 64 : 128;
+    static constexpr int kStages = 4;
+    static constexpr int kSmem = kStages * kStage + 16;  // + two mbarriers
 };
 
 // Instruction descriptor of kind::f16 with both operands MN-major.
@@ -796,49 +919,58 @@ __host__ __device__ constexpr uint32_t mma_idesc_mn(int M, int N) {
     return mma_idesc(M, N) | (1u << 15) | (1u << 16);
 }
 
-constexpr int kWgThreads = 2 * kTile;  // two threads per staged position: each stages half the planes
+constexpr int kWgSplit = 4;                   // threads per staged position, each with a share of the planes
+constexpr int kWgThreads = kWgSplit * kTile;
+
+// Position q of the bands: `at` = padded position s0 - P - 1 + q as row and
+// column; band dy is dy rows further down.
+template <int CCH>
+__device__ __forceinline__ void wgrad_stage_bands(const bf16* __restrict__ x, const Geom& g, int64_t pbase, PosRC at,
+                                                  uint32_t dst, int share) {
+    using W = WgradTc<CCH, 16>;
+    const bool in_row = at.c >= 1 && at.c <= g.W;
+    const int pix0 = at.r * g.W + at.c - 1;
+#pragma unroll
+    for (int pl = 0; pl < 3 * CCH; ++pl) {
+        const int dy = pl / CCH, c = pl - dy * CCH;
+        if ((CCH > 1 ? c : dy) != share) continue;
+        const bool valid = in_row && at.r + dy >= 0 && at.r + dy < g.H;
+        const bf16* src = valid ? x + ((pbase + pix0 + dy * g.W) * CCH + c) * 8 : x;
+        cp_async16(dst + pl * W::kAPlane, src, valid);
+    }
+}
 
 template <int CCH, int NOUT, int CIN, int COUT, class TDY>
 __device__ __forceinline__ void wgrad_stage(const bf16* __restrict__ x, const TDY* __restrict__ dy, const Geom& g,
                                             int64_t pbase, int s0, unsigned char* buf) {
     using W = WgradTc<CCH, NOUT>;
-    const int q = threadIdx.x & (kTile - 1), half = threadIdx.x / kTile;
+    const int q = threadIdx.x & (kTile - 1), share = threadIdx.x / kTile;
     const uint32_t a = smem_u32(buf);
-    const PosRC base = position_rc(g, s0 - g.P - 1 + q);  // tap (0, 0) of output position s0 + q
-#pragma unroll 1
-    for (int pl = half; pl < W::kDataPlanes; pl += 2) {
-        const int tap = pl / CCH, c = pl - tap * CCH;
-        const int pix = rc_pixel(g, rc_add(g, base, tap / 3, tap % 3));
-        const bf16* src = pix >= 0 ? x + ((pbase + pix) * CCH + c) * 8 : x;
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(a + pl * W::kPlane + q * 16), "l"(src),
-                     "r"(pix >= 0 ? 16 : 0)
-                     : "memory");
-    }
+    const PosRC base = position_rc(g, s0 - g.P - 1 + q);
+    wgrad_stage_bands<CCH>(x, g, pbase, base, a + q * 16, share);
+    if (q < 2)  // positions 128 and 129
+        wgrad_stage_bands<CCH>(x, g, pbase, rc_add(g, base, g.step_r, g.step_c), a + (kTile + q) * 16, share);
     const int pix = rc_pixel(g, rc_add(g, base, 1, 1));  // output position s0 + q
-    const uint32_t b = a + W::kAPlanes * W::kPlane;
+    const uint32_t b = a + W::kAPlanes * W::kAPlane;
     if constexpr (sizeof(TDY) == 2) {
 #pragma unroll
-        for (int c = half; c < W::kBPlanes; c += 2) {
-            const TDY* src = pix >= 0 ? dy + (pbase + pix) * COUT + c * 8 : dy;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(b + c * W::kPlane + q * 16),
-                         "l"(src), "r"(pix >= 0 ? 16 : 0)
-                         : "memory");
+        for (int c = 0; c < W::kBPlanes; ++c) {
+            if (c != share) continue;
+            cp_async16(b + c * W::kBPlane + q * 16, pix >= 0 ? dy + (pbase + pix) * COUT + c * 8 : dy, pix >= 0);
         }
-    } else if (half == 0) {  // one FP32 channel -> BF16 hi in column 0, lo in column 1
+    } else if (share == 0) {  // one FP32 channel -> BF16 hi in column 0, lo in column 1
         const float d = pix >= 0 ? to_f(dy[pbase + pix]) : 0.f;
         const bf16 hi = __float2bfloat16(d);
         const bf16 lo = __float2bfloat16(d - __bfloat162float(hi));
         __nv_bfloat162 pr;
         pr.x = hi;
         pr.y = lo;
-        *reinterpret_cast<uint4*>(buf + W::kAPlanes * W::kPlane + q * 16) =
+        *reinterpret_cast<uint4*>(buf + W::kAPlanes * W::kAPlane + q * 16) =
             make_uint4(*reinterpret_cast<const uint32_t*>(&pr), 0u, 0u, 0u);
-    } else {
-#pragma unroll
-        for (int c = 1; c < W::kBPlanes; ++c)
-            *reinterpret_cast<uint4*>(buf + (W::kAPlanes + c) * W::kPlane + q * 16) = make_uint4(0u, 0u, 0u, 0u);
+    } else if (share < W::kBPlanes) {
+        *reinterpret_cast<uint4*>(buf + W::kAPlanes * W::kAPlane + share * W::kBPlane + q * 16) =
+            make_uint4(0u, 0u, 0u, 0u);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
 template <int CCH, int NOUT, int CIN, int COUT, class TDY>
@@ -849,16 +981,16 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16* __restrict_
     constexpr int K = kTaps * CIN;
     constexpr int NV = (K + 1) * COUT;
     extern __shared__ __align__(1024) unsigned char sm[];
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + 2 * W::kStage);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + W::kStages * W::kStage);
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // constant planes of both stages: the ones plane (bias row) and zeros up
+    // constant planes of every stage: the ones plane (bias row) and zeros up
     // to the M tile boundary; staging never writes them
-    for (int st = 0; st < 2; ++st)
-        for (int pl = W::kDataPlanes + tid / kTile; pl < W::kAPlanes; pl += kWgThreads / kTile) {
-            const uint32_t one = pl == W::kDataPlanes ? 0x3F803F80u : 0u;  // BF16 1.0 pairs
-            *reinterpret_cast<uint4*>(sm + st * W::kStage + pl * W::kPlane + (tid & (kTile - 1)) * 16) =
+    for (int st = 0; st < W::kStages; ++st)
+        for (int q = tid; q < (W::kAPlanes - W::kDataPlanes) * W::kPos; q += kWgThreads) {
+            const uint32_t one = q < W::kPos ? 0x3F803F80u : 0u;  // BF16 1.0 pairs
+            *reinterpret_cast<uint4*>(sm + st * W::kStage + W::kDataPlanes * W::kAPlane + q * 16) =
                 make_uint4(one, one, one, one);
         }
     if (warp == 0) {
@@ -867,87 +999,88 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16* __restrict_
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) mbar_init(smem_u32(mbar), 1);
+    if (tid < 2) mbar_init(smem_u32(mbar + tid), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
     constexpr uint32_t idesc = mma_idesc_mn(kTile, NOUT);
-    uint32_t phase = 0;
-    int buf = 0;
-    bool any = false, failed = false;
+    bool failed = false;
     long long wait_polls = first_wait;
+    const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // this CTA's tiles, >= 1
 
-    int64_t tile = blockIdx.x;
-    if (tile < ntiles) {
-        int64_t pb;
-        int s0;
-        tile_origin(tile, g, pb, s0);
-        wgrad_stage<CCH, NOUT, CIN, COUT, TDY>(x, dy, g, pb, s0, sm);
-    }
-    for (; tile < ntiles; tile += gridDim.x) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    TileWalk ahead(g);
+    auto stage = [&](int i) {  // the CTA's next tile, its i-th, into its stage (an empty group past the end)
+        if (i < mine) {
+            wgrad_stage<CCH, NOUT, CIN, COUT, TDY>(x, dy, g, ahead.pixel, ahead.s0,
+                                                   sm + (i % W::kStages) * W::kStage);
+            ahead.step(g);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // Two tiles' MMAs may be in flight: tile i's complete on barrier i & 1, and
+    // are waited for two tiles later, when tile i + 4 is about to take their
+    // stage's place. (Waiting for tile i - 1 before issuing tile i left the
+    // tensor core idle for every issue and completion: 128 us, 119 us with two in flight.)
+    stage(0);
+    stage(1);
+    for (int i = 0; i < mine + 2; ++i) {
+        // tile i has landed, the MMAs of tile i - 2 are complete
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t base = smem_u32(sm + buf * W::kStage);
-            const uint32_t bb = base + W::kAPlanes * W::kPlane;
-#pragma unroll 1
-            for (int ks = 0; ks < kTile / 16; ++ks)
-#pragma unroll
-                for (int mt = 0; mt < W::MT; ++mt) {
-                    // MN-major, no swizzle: element (mn, k) at start + (mn / 8) * SBO + (mn % 8) * 2
-                    // + (k / 8) * LBO + (k % 8) * 16, with SBO = one plane and LBO = 8 positions
-                    const uint64_t ad = smem_desc(base + mt * 16 * W::kPlane + ks * 256, 128, W::kPlane);
-                    const uint64_t bd = smem_desc(bb + ks * 256, 128, W::kPlane);
-                    mma_bf16(tmem + mt * NOUT, ad, bd, idesc, (any || ks > 0) ? 1u : 0u);
-                }
-            mma_commit(smem_u32(mbar));
+        bool ok = true;
+        if (i >= 2) {
+            ok = mbar_wait(smem_u32(mbar + (i & 1)), (uint32_t)((i - 2) >> 1) & 1u, wait_polls);
+            wait_polls = kWaitLimit;
         }
-        any = true;
-        const int64_t next = tile + gridDim.x;
-        if (next < ntiles) {  // stage the next tile while these MMAs run
-            int64_t pb;
-            int s1;
-            tile_origin(next, g, pb, s1);
-            wgrad_stage<CCH, NOUT, CIN, COUT, TDY>(x, dy, g, pb, s1, sm + (buf ^ 1) * W::kStage);
-        }
-        __syncwarp();
-        const bool ok = __syncthreads_and(mbar_wait(smem_u32(mbar), phase, wait_polls));
-        wait_polls = kWaitLimit;
-        phase ^= 1u;
-        if (!ok) {
+        if (!__syncthreads_and(ok)) {
             if (tid == 0) atomicExch(err, 1);
-            // the MMAs in flight get a bounded chance to land before the
-            // tensor memory is released
-            mbar_wait(smem_u32(mbar), phase ^ 1u, kWaitLimit);
+            // the MMAs in flight (tiles i - 2 and i - 1) get a bounded chance
+            // to land before the tensor memory is released
+            for (int q = i - 2; q < i && q < mine; ++q)
+                mbar_wait(smem_u32(mbar + (q & 1)), (uint32_t)(q >> 1) & 1u, kWaitLimit);
             failed = true;
             break;
         }
-        buf ^= 1;
+        if (i < mine && tid == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // MN-major, no swizzle: element (mn, k) at start + (mn / 8) * SBO + (mn % 8) * 2
+            // + (k / 8) * LBO + (k % 8) * 16, with SBO = one plane and LBO = 8 positions; the
+            // starts (16-byte units, the descriptor's low bits) advance 16 positions a K step
+            // and one position a tap column
+            const uint32_t base = smem_u32(sm + (i % W::kStages) * W::kStage);
+            const uint64_t ad = smem_desc(base, 128, W::kAPlane);
+            const uint64_t bd = smem_desc(base + W::kAPlanes * W::kAPlane, 128, W::kBPlane);
+#pragma unroll
+            for (int ks = 0; ks < kTile / 16; ++ks)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx)
+                    mma_bf16(tmem + dx * NOUT, ad + ks * 16 + dx, bd + ks * 16, idesc, (i > 0 || ks > 0) ? 1u : 0u);
+            mma_commit(smem_u32(mbar + (i & 1)));
+        }
+        __syncwarp();
+        stage(i + 2);  // into the stage that tile i - 2 used
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (any && !failed) {
+    if (!failed) {
         float* out = part + (int64_t)blockIdx.x * NV;
-        // warp w reads tensor-memory lanes 32 (w % 4) .. + 31; the two groups of
-        // four warps take alternate M tiles
+        // warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (row r = (plane, channel) of the chunk);
+        // group of four warps dx reads tap column dx's accumulator
         const int sub = warp & 3, group = warp >> 2;
-        const int r = sub * 32 + lane;  // row of D (tensor-memory lane)
-#pragma unroll 1
-        for (int mt = group; mt < W::MT; mt += kWgThreads / 128) {
+        const int r = sub * 32 + lane, pl = r / 8, e = r % 8;
+        const int dy_tap = pl / CCH, ci = (pl - dy_tap * CCH) * 8 + e;
+        if (group < 3) {
+            const int dx = group;
             float v[32];
-            tmem_ld32(tmem + ((uint32_t)(sub * 32) << 16) + mt * NOUT, v);
-            const int pl = mt * 16 + r / 8, e = r % 8;
+            tmem_ld32(tmem + ((uint32_t)(sub * 32) << 16) + dx * NOUT, v);
             int k = -1;
             if (pl < W::kDataPlanes) {
-                const int tap = pl / CCH, ci = (pl - tap * CCH) * 8 + e;
-                if (ci < CIN) k = tap * CIN + ci;
-            } else if (pl == W::kDataPlanes && e == 0) {
+                if (ci < CIN) k = (dy_tap * 3 + dx) * CIN + ci;
+            } else if (pl == W::kDataPlanes && e == 0 && dx == 0) {
                 k = K;  // the ones plane: bias gradient
             }
             if (k >= 0) {
@@ -1253,7 +1386,7 @@ void wgrad(dgpu_net* N, const bf16* x, const TDY* dy, int64_t count, int layer) 
     const int64_t ntiles = count * N->g.tiles_per_img;
     int ctas;
     if (N->engine == DGPU_NET_TENSOR) {
-        // tensor cores: one CTA per SM (two ~100 KB stages of shared memory)
+        // tensor cores: one CTA per SM (four 43 KB stages of shared memory)
         constexpr int CCH = XS / 8;
         constexpr int NOUT = COUT == 1 ? 16 : COUT;
         using W = WgradTc<CCH, NOUT>;
@@ -1268,7 +1401,7 @@ void wgrad(dgpu_net* N, const bf16* x, const TDY* dy, int64_t count, int layer) 
                                                                                                   ntiles, N->gpart.p);
     }
     launched(N);
-    k_reduce_wgrad<<<grid_for(WG::NV, 256, N->sms), 256, 0, N->stream>>>(
+    k_reduce_wgrad<<<(WG::NV + 31) / 32, 256, 0, N->stream>>>(
         N->gpart.p, ctas, WG::NV, WG::K, N->grad.p + N->T.off_w[layer], N->grad.p + N->T.off_b[layer]);
     launched(N);
 }
@@ -1281,7 +1414,7 @@ void backward(dgpu_net* N, int64_t count, float* loss_slot) {
                                                                     N->g.H, N->g.W, (int)count, N->err_e.p,
                                                                     N->dout.p, N->loss_part.p);
         launched(N);
-        k_mean_parts<<<1, 32, 0, N->stream>>>(N->loss_part.p, (int)count, loss_slot);
+        k_mean_parts<<<1, kEnergyThreads, 0, N->stream>>>(N->loss_part.p, (int)count, loss_slot);
         launched(N);
     } else {
         k_mse<<<kLossBlocks, kLossThreads, 0, N->stream>>>(N->out.p, N->target.p, npix, N->dout.p,
@@ -1293,9 +1426,8 @@ void backward(dgpu_net* N, int64_t count, float* loss_slot) {
     // output layer (32 -> 1): weight gradient, then the input gradient through
     // the GELU of layer 4 (a 1 -> 32 convolution with the flipped weights)
     wgrad<float, 32, 32, 1>(N, N->act[4].p, N->dout.p, count, 5);
-    k_conv_simt<float, 1><<<grid_for(npix * kC, 256, N->sms), 256, 0, N->stream>>>(
-        N->dout.p, wt(N, 5), nullptr, kC, N->g.H, N->g.W, npix, kEpiGeluGrad, N->pre[4].p, nullptr, N->dpre[0].p,
-        nullptr);
+    k_out_dgrad<<<grid_for(npix * 4, 256, N->sms), 256, 0, N->stream>>>(N->dout.p, wt(N, 5), N->g.H, N->g.W, npix,
+                                                                        N->pre[4].p, N->dpre[0].p);
     launched(N);
     int cur = 0;  // dpre[cur] holds the gradient at layer l's pre-activation
     for (int l = 4; l >= 1; --l) {
@@ -1482,8 +1614,8 @@ int tc_grid(dgpu_net* N, std::string* info) {
     const int by_smem = smem_sm / (smem + (int)fa.sharedSizeBytes + reserved);
     const int by_regs = regs_sm / std::max(1, fa.numRegs * kConvThreads);
     const int by_thr = thr_sm / kConvThreads;
-    const int manual = std::min(std::min(by_smem, by_regs), std::min(by_thr, 16));  // 16 x 32 TMEM columns
-    const int per_sm = std::max(1, std::max(api, manual));
+    const int manual = std::min(std::min(by_smem, by_regs), std::min(by_thr, 512 / kConvCols));  // 512 tensor-memory columns an SM
+    const int per_sm = std::max(1, std::min(std::max(api, manual), 512 / kConvCols));
     char buf[200];
     std::snprintf(buf, sizeof buf, "tc<%d,%d>: smem %d B, %d regs, occupancy api %d / resources %d -> %d CTAs/SM; ",
                   CCH, NOUT, smem + (int)fa.sharedSizeBytes, fa.numRegs, api, manual, per_sm);
