@@ -81,36 +81,52 @@ __device__ __forceinline__ void df_axpy(DF& s, float ch, float cl, float x, floa
 }
 
 // -------------------------------------------------------------- staging
+//
+// A thread's cells are all loaded before any of them is stored to shared
+// memory: a tile's halo has up to 384 cells for 256 threads, and one cell at a
+// time (load, store, load, store) cost a second L2 round trip on the way from
+// one visit to the next.
+
+constexpr int kVisitThreads = 256;
 
 template <class T, int TH, int TW, int R, bool WITH_D, bool WITH_LO>
 __device__ __forceinline__ void stage_coeffs(const VisitLevel<T>& V, int ti0, int tj0, T* es, T* ns, T* ds, T* is,
                                              T* elo, T* nlo, T* dlo) {
     using G = Tile<TH, TW, R>;
+    constexpr int kIter = (G::S + kVisitThreads - 1) / kVisitThreads;
     const int n = V.n;
-    for (int q = threadIdx.x; q < G::S; q += blockDim.x) {
+    T ev[kIter], nv[kIter], dv[kIter], iv[kIter], el[kIter], nl[kIter], dl[kIter];
+#pragma unroll
+    for (int u = 0; u < kIter; ++u) {
+        const int q = threadIdx.x + u * kVisitThreads;
         const int li = q / G::SW, lj = q - li * G::SW;
         const int gi = ti0 - R + li, gj = tj0 - R + lj;
-        T ev = T(0), nv = T(0), dv = T(0), iv = T(0), el = T(0), nl = T(0), dl = T(0);
-        if (gi >= 0 && gi < n && gj >= 0 && gj < n) {
+        ev[u] = nv[u] = dv[u] = iv[u] = el[u] = nl[u] = dl[u] = T(0);
+        if (q < G::S && gi >= 0 && gi < n && gj >= 0 && gj < n) {
             const int k = gi * n + gj;
-            ev = __ldg(V.e + k);
-            nv = __ldg(V.nf + k);
-            if (WITH_D) dv = __ldg(V.d + k);
-            iv = __ldg(V.id + k);
+            ev[u] = __ldg(V.e + k);
+            nv[u] = __ldg(V.nf + k);
+            if (WITH_D) dv[u] = __ldg(V.d + k);
+            iv[u] = __ldg(V.id + k);
             if (WITH_LO) {
-                el = __ldg(V.elo + k);
-                nl = __ldg(V.nlo + k);
-                if (WITH_D) dl = __ldg(V.dlo + k);
+                el[u] = __ldg(V.elo + k);
+                nl[u] = __ldg(V.nlo + k);
+                if (WITH_D) dl[u] = __ldg(V.dlo + k);
             }
         }
-        es[q] = ev;
-        ns[q] = nv;
-        if (WITH_D) ds[q] = dv;
-        is[q] = iv;
+    }
+#pragma unroll
+    for (int u = 0; u < kIter; ++u) {
+        const int q = threadIdx.x + u * kVisitThreads;
+        if (q >= G::S) break;
+        es[q] = ev[u];
+        ns[q] = nv[u];
+        if (WITH_D) ds[q] = dv[u];
+        is[q] = iv[u];
         if (WITH_LO) {
-            elo[q] = el;
-            nlo[q] = nl;
-            if (WITH_D) dlo[q] = dl;
+            elo[q] = el[u];
+            nlo[q] = nl[u];
+            if (WITH_D) dlo[q] = dl[u];
         }
     }
 }
@@ -120,30 +136,40 @@ template <class T, int TH, int TW, int R>
 __device__ __forceinline__ void stage_vectors(const VisitLevel<T>& V, const T* __restrict__ xin,
                                               const T* __restrict__ xc, int ti0, int tj0, T* xs, T* bs, T* bls) {
     using G = Tile<TH, TW, R>;
+    constexpr int kIter = (G::S + kVisitThreads - 1) / kVisitThreads;
     const int n = V.n, nc = (n + 1) >> 1;
-    for (int q = threadIdx.x; q < G::S; q += blockDim.x) {
+    T xv[kIter], cv[kIter], bv[kIter], bl[kIter];
+#pragma unroll
+    for (int u = 0; u < kIter; ++u) {
+        const int q = threadIdx.x + u * kVisitThreads;
         const int li = q / G::SW, lj = q - li * G::SW;
         const int gi = ti0 - R + li, gj = tj0 - R + lj;
-        T xv = T(0), bv = T(0), bl = T(0);
-        if (gi >= 0 && gi < n && gj >= 0 && gj < n) {
+        xv[u] = cv[u] = bv[u] = bl[u] = T(0);
+        if (q < G::S && gi >= 0 && gi < n && gj >= 0 && gj < n) {
             const int k = gi * n + gj;
-            if (xin) xv = xin[k];
-            if (xc) xv += xc[(gi >> 1) * nc + (gj >> 1)];
-            bv = V.b[k];
-            if (bls && V.blo) bl = V.blo[k];
+            if (xin) xv[u] = xin[k];
+            if (xc) cv[u] = xc[(gi >> 1) * nc + (gj >> 1)];
+            bv[u] = V.b[k];
+            if (bls && V.blo) bl[u] = V.blo[k];
         }
-        xs[q] = xv;
-        bs[q] = bv;
-        if (bls) bls[q] = bl;
+    }
+#pragma unroll
+    for (int u = 0; u < kIter; ++u) {
+        const int q = threadIdx.x + u * kVisitThreads;
+        if (q >= G::S) break;
+        xs[q] = xc ? xv[u] + cv[u] : xv[u];
+        bs[q] = bv[u];
+        if (bls) bls[q] = bl[u];
     }
 }
 
 // One colour pass over the in-domain cells of colour c inside local rows /
 // cols [LO, S-LO): every row of the region holds exactly half its cells of
 // each colour (the staged width is even), so cells are enumerated directly.
+// `zero`: the iterate is zero, x = b / d (the same bits as adding e * 0).
 template <class T, int TH, int TW, int R, int LO>
 __device__ __forceinline__ void stage_gs(int n, int ti0, int tj0, int c, T* xs, const T* es, const T* ns,
-                                         const T* is, const T* bs) {
+                                         const T* is, const T* bs, bool zero = false) {
     using G = Tile<TH, TW, R>;
     constexpr int h = G::SH - 2 * LO, hw = (G::SW - 2 * LO) / 2;
     static_assert((G::SW - 2 * LO) % 2 == 0, "even staged width");
@@ -158,11 +184,71 @@ __device__ __forceinline__ void stage_gs(int n, int ti0, int tj0, int c, T* xs, 
         if (gi < 0 || gi >= n || gj < 0 || gj >= n) continue;
         const int s = li * G::SW + lj;
         T v = bs[s];
-        v += es[s] * xs[s + 1];
-        v += es[s - 1] * xs[s - 1];
-        v += ns[s] * xs[s + G::SW];
-        v += ns[s - G::SW] * xs[s - G::SW];
+        if (!zero) {
+            v += es[s] * xs[s + 1];
+            v += es[s - 1] * xs[s - 1];
+            v += ns[s] * xs[s + G::SW];
+            v += ns[s - G::SW] * xs[s - G::SW];
+        }
         xs[s] = v * is[s];
+    }
+}
+
+// The restricted residual of the tile (level.hpp:122-137, :214-227), four
+// threads an aggregate, one per cell: each forms its cell's terms, the sums run
+// over the four in the order of one thread doing all of them (same bits; cells
+// outside the domain contribute zero). One thread an aggregate left one warp
+// of the CTA with all of this, at the end of the chain from visit to visit
+// (with the staging above: 1024^2 mixed 232 -> 208 us an iteration, FP64 335 ->
+// 293 us).
+template <class T, int TH, int TW, int R>
+__device__ __forceinline__ void stage_residual(int n, int ti0, int tj0, const T* xs, const T* es, const T* ns,
+                                               const T* ds, const T* bs, const T* elo, const T* nlo, const T* dlo,
+                                               const T* bls, T* bc) {
+    using G = Tile<TH, TW, R>;
+    const int nc = (n + 1) >> 1;
+    static_assert((TH * TW) % 32 == 0, "whole warps");
+#pragma unroll 1
+    for (int t = threadIdx.x; t < TH * TW; t += kVisitThreads) {
+        const int agg = t >> 2, cell = t & 3, ai = agg / (TW / 2), aj = agg - ai * (TW / 2);
+        const int I = (ti0 >> 1) + ai, J = (tj0 >> 1) + aj;
+        const int s = (R + 2 * ai + (cell >> 1)) * G::SW + (R + 2 * aj + (cell & 1));
+        const bool inside = 2 * I + (cell >> 1) < n && 2 * J + (cell & 1) < n;
+        if constexpr (sizeof(T) == 8) {
+            T v = fma(ds[s], xs[s], -__dmul_rn(es[s], xs[s + 1]));  // which product rounds alone is fixed here
+            v = fma(-es[s - 1], xs[s - 1], v);
+            v = fma(-ns[s], xs[s + G::SW], v);
+            v = fma(-ns[s - G::SW], xs[s - G::SW], v);
+            const T r = inside ? bs[s] - v : T(0);
+            T acc = __shfl_sync(0xffffffffu, r, 0, 4);
+            acc += __shfl_sync(0xffffffffu, r, 1, 4);
+            acc += __shfl_sync(0xffffffffu, r, 2, 4);
+            acc += __shfl_sync(0xffffffffu, r, 3, 4);
+            if (cell == 0 && I < nc && J < nc) bc[I * nc + J] = acc;
+        } else {
+            // r = b - d x + e xE + w xW + n xN + s xS as (hi, lo) terms
+            float vh[6], vl[6];
+            auto term = [&](int k, float ch, float cl, float x, float sign) {
+                const float p = ch * x;
+                const float pe = fmaf(ch, x, -p);
+                vh[k] = inside ? sign * p : 0.f;
+                vl[k] = inside ? sign * (pe + cl * x) : 0.f;
+            };
+            vh[0] = inside ? bs[s] : 0.f;
+            vl[0] = inside ? bls[s] : 0.f;
+            term(1, ds[s], dlo[s], xs[s], -1.f);
+            term(2, es[s], elo[s], xs[s + 1], 1.f);
+            term(3, es[s - 1], elo[s - 1], xs[s - 1], 1.f);
+            term(4, ns[s], nlo[s], xs[s + G::SW], 1.f);
+            term(5, ns[s - G::SW], nlo[s - G::SW], xs[s - G::SW], 1.f);
+            DF acc{0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int k = 0; k < 6; ++k)
+                    df_add(acc, __shfl_sync(0xffffffffu, vh[k], c, 4), __shfl_sync(0xffffffffu, vl[k], c, 4));
+            if (cell == 0 && I < nc && J < nc) bc[I * nc + J] = acc.hi + acc.lo;
+        }
     }
 }
 
@@ -180,7 +266,7 @@ struct PostSmem {
 // Pre-smoothing (1 sweep: red then black), residual, restriction. xin == null
 // means the iterate is known to be zero (first call from the parent).
 template <class T, int TH, int TW>
-__global__ void __launch_bounds__(256) k_visit_pre(VisitLevel<T> V, const T* __restrict__ xin, T* __restrict__ xout,
+__global__ void __launch_bounds__(kVisitThreads) k_visit_pre(VisitLevel<T> V, const T* __restrict__ xin, T* __restrict__ xout,
                                                    T* __restrict__ bc) {
     constexpr int R = 3;
     constexpr bool LO = sizeof(T) == 4;
@@ -196,7 +282,7 @@ __global__ void __launch_bounds__(256) k_visit_pre(VisitLevel<T> V, const T* __r
     T* nlo = LO ? elo + G::S : nullptr;
     T* dlo = LO ? nlo + G::S : nullptr;
     T* bls = LO ? dlo + G::S : nullptr;
-    const int n = V.n, nc = (n + 1) >> 1;
+    const int n = V.n;
     const int tiles_x = (n + TW - 1) / TW, tiles = tiles_x * ((n + TH - 1) / TH);
     bool waited = false;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -208,50 +294,11 @@ __global__ void __launch_bounds__(256) k_visit_pre(VisitLevel<T> V, const T* __r
         }
         stage_vectors<T, TH, TW, R>(V, xin, nullptr, ti0, tj0, xs, bs, bls);
         __syncthreads();
-        stage_gs<T, TH, TW, R, 1>(n, ti0, tj0, 0, xs, es, ns, is, bs);  // red, rings <= 2
+        stage_gs<T, TH, TW, R, 1>(n, ti0, tj0, 0, xs, es, ns, is, bs, !xin);  // red, rings <= 2
         __syncthreads();
         stage_gs<T, TH, TW, R, 2>(n, ti0, tj0, 1, xs, es, ns, is, bs);  // black, rings <= 1
         __syncthreads();
-        // residual of each tile cell, summed per aggregate (level.hpp:122-137, :214-227)
-        for (int q = threadIdx.x; q < (TH / 2) * (TW / 2); q += blockDim.x) {
-            const int ai = q / (TW / 2), aj = q - ai * (TW / 2);
-            const int I = (ti0 >> 1) + ai, J = (tj0 >> 1) + aj;
-            if (I >= nc || J >= nc) continue;
-            if constexpr (sizeof(T) == 8) {
-                T acc = T(0);
-                for (int di = 0; di < 2; ++di) {
-                    if (2 * I + di >= n) break;
-                    for (int dj = 0; dj < 2; ++dj) {
-                        if (2 * J + dj >= n) break;
-                        const int s = (R + 2 * ai + di) * G::SW + (R + 2 * aj + dj);
-                        T v = ds[s] * xs[s];
-                        v -= es[s] * xs[s + 1];
-                        v -= es[s - 1] * xs[s - 1];
-                        v -= ns[s] * xs[s + G::SW];
-                        v -= ns[s - G::SW] * xs[s - G::SW];
-                        acc += bs[s] - v;
-                    }
-                }
-                bc[I * nc + J] = acc;
-            } else {
-                DF acc{0.f, 0.f};
-                for (int di = 0; di < 2; ++di) {
-                    if (2 * I + di >= n) break;
-                    for (int dj = 0; dj < 2; ++dj) {
-                        if (2 * J + dj >= n) break;
-                        const int s = (R + 2 * ai + di) * G::SW + (R + 2 * aj + dj);
-                        // r = b - d x + e xE + w xW + n xN + s xS
-                        df_add(acc, bs[s], bls[s]);
-                        df_axpy(acc, ds[s], dlo[s], xs[s], -1.f);
-                        df_axpy(acc, es[s], elo[s], xs[s + 1], 1.f);
-                        df_axpy(acc, es[s - 1], elo[s - 1], xs[s - 1], 1.f);
-                        df_axpy(acc, ns[s], nlo[s], xs[s + G::SW], 1.f);
-                        df_axpy(acc, ns[s - G::SW], nlo[s - G::SW], xs[s - G::SW], 1.f);
-                    }
-                }
-                bc[I * nc + J] = acc.hi + acc.lo;
-            }
-        }
+        stage_residual<T, TH, TW, R>(n, ti0, tj0, xs, es, ns, ds, bs, elo, nlo, dlo, bls, bc);
         // the smoothed iterate of the tile
         for (int q = threadIdx.x; q < TH * TW; q += blockDim.x) {
             const int li = q / TW, lj = q - li * TW;
@@ -275,7 +322,7 @@ struct MidSmem {
 };
 
 template <class T, int TH, int TW>
-__global__ void __launch_bounds__(256) k_visit_mid(VisitLevel<T> V, const T* __restrict__ xin,
+__global__ void __launch_bounds__(kVisitThreads) k_visit_mid(VisitLevel<T> V, const T* __restrict__ xin,
                                                    const T* __restrict__ xc, T* __restrict__ xout,
                                                    T* __restrict__ bc) {
     constexpr int R = 4;
@@ -292,7 +339,7 @@ __global__ void __launch_bounds__(256) k_visit_mid(VisitLevel<T> V, const T* __r
     T* nlo = LO ? elo + G::S : nullptr;
     T* dlo = LO ? nlo + G::S : nullptr;
     T* bls = LO ? dlo + G::S : nullptr;
-    const int n = V.n, nc = (n + 1) >> 1;
+    const int n = V.n;
     const int tiles_x = (n + TW - 1) / TW, tiles = tiles_x * ((n + TH - 1) / TH);
     bool waited = false;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -310,44 +357,7 @@ __global__ void __launch_bounds__(256) k_visit_mid(VisitLevel<T> V, const T* __r
         __syncthreads();
         stage_gs<T, TH, TW, R, 3>(n, ti0, tj0, 1, xs, es, ns, is, bs);  // pre black, rings <= 1
         __syncthreads();
-        for (int q = threadIdx.x; q < (TH / 2) * (TW / 2); q += blockDim.x) {
-            const int ai = q / (TW / 2), aj = q - ai * (TW / 2);
-            const int I = (ti0 >> 1) + ai, J = (tj0 >> 1) + aj;
-            if (I >= nc || J >= nc) continue;
-            if constexpr (sizeof(T) == 8) {
-                T acc = T(0);
-                for (int di = 0; di < 2; ++di) {
-                    if (2 * I + di >= n) break;
-                    for (int dj = 0; dj < 2; ++dj) {
-                        if (2 * J + dj >= n) break;
-                        const int s = (R + 2 * ai + di) * G::SW + (R + 2 * aj + dj);
-                        T v = ds[s] * xs[s];
-                        v -= es[s] * xs[s + 1];
-                        v -= es[s - 1] * xs[s - 1];
-                        v -= ns[s] * xs[s + G::SW];
-                        v -= ns[s - G::SW] * xs[s - G::SW];
-                        acc += bs[s] - v;
-                    }
-                }
-                bc[I * nc + J] = acc;
-            } else {
-                DF acc{0.f, 0.f};
-                for (int di = 0; di < 2; ++di) {
-                    if (2 * I + di >= n) break;
-                    for (int dj = 0; dj < 2; ++dj) {
-                        if (2 * J + dj >= n) break;
-                        const int s = (R + 2 * ai + di) * G::SW + (R + 2 * aj + dj);
-                        df_add(acc, bs[s], bls[s]);
-                        df_axpy(acc, ds[s], dlo[s], xs[s], -1.f);
-                        df_axpy(acc, es[s], elo[s], xs[s + 1], 1.f);
-                        df_axpy(acc, es[s - 1], elo[s - 1], xs[s - 1], 1.f);
-                        df_axpy(acc, ns[s], nlo[s], xs[s + G::SW], 1.f);
-                        df_axpy(acc, ns[s - G::SW], nlo[s - G::SW], xs[s - G::SW], 1.f);
-                    }
-                }
-                bc[I * nc + J] = acc.hi + acc.lo;
-            }
-        }
+        stage_residual<T, TH, TW, R>(n, ti0, tj0, xs, es, ns, ds, bs, elo, nlo, dlo, bls, bc);
         for (int q = threadIdx.x; q < TH * TW; q += blockDim.x) {
             const int li = q / TW, lj = q - li * TW;
             const int gi = ti0 + li, gj = tj0 + lj;
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(256) k_visit_mid(VisitLevel<T> V, const T* __r
 // Prolongation + post-smoothing (1 sweep: black then red). On level 0 (r
 // given) also r . z and beta, like k_gs0_dot.
 template <class T, int TH, int TW>
-__global__ void __launch_bounds__(256) k_visit_post(VisitLevel<T> V, const T* __restrict__ xin,
+__global__ void __launch_bounds__(kVisitThreads) k_visit_post(VisitLevel<T> V, const T* __restrict__ xin,
                                                     const T* __restrict__ xc, T* __restrict__ xout,
                                                     const double* __restrict__ r, CgState* st, double* partials) {
     constexpr int R = 2;

@@ -823,11 +823,10 @@ static inline int tiles_grid(int n) {
     return (int)(t < kMaxTileGrid ? t : kMaxTileGrid);
 }
 
-// Threads of a visit CTA. 256 for both tile shapes: measured at 1024^2
-// (mixed / FP64) 35.0 / 42.7 ms with 128 threads on the 8 x 16 tiles, 32.8 /
-// 39.5 ms with 256 (more loads in flight while the halo is staged), 33.1 /
-// 40.9 ms with 512; 512 on the 16 x 32 tiles measured slower as well.
-constexpr int kVisitThreads = 256;
+// Threads of a visit CTA (kVisitThreads): 256 for both tile shapes. Measured at
+// 1024^2 (mixed / FP64) 35.0 / 42.7 ms with 128 threads on the 8 x 16 tiles,
+// 32.8 / 39.5 ms with 256 (more loads in flight while the halo is staged), 33.1
+// / 40.9 ms with 512; 512 on the 16 x 32 tiles measured slower as well.
 template <class T>
 void launch_visit_pre(const VisitLevel<T>& V, const T* xin, T* xout, T* bc, cudaStream_t s) {
     if (V.n <= 256)
