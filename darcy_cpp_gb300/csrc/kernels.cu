@@ -256,6 +256,218 @@ __global__ void k_prolong_gs1(Lvl<T> L, const T* xc, const CgState* st) {
     prolong_gs1<GridScope>(L, xc);
 }
 
+// The same level operations for an even side, one thread per 2 x 2 aggregate:
+// no index division, two cells of a colour (or four residuals) share their
+// loads, rows read as pairs, and only the four neighbours outside the
+// aggregate need a boundary test (an absent one enters as e * 0). Arithmetic
+// and order as gs_colour, cell_residual and prolong_gs1, which odd sides keep
+// (their rows have no aligned pairs): the same bits. Bound by HBM (FP32) and
+// the FP64 pipe. us a launch on GB300 at 2048^2, one cell a thread -> here:
+//                               FP64           FP32
+//   red, zero start          10.7 ->  9.6    6.7 ->  5.4
+//   black                    32.6 -> 32.2   11.0 ->  8.2
+//   residual + restriction   59.3 -> 51.6   34.5 -> 24.3  (double-float)
+//   prolongation + black     40.9 -> 36.1   16.0 ->  9.6
+// An even side always takes these: at every size measured (64 up) none is slower.
+constexpr int kAggX = 32, kAggY = 8;  // aggregates a CTA covers
+static dim3 agg_grid(int n) { return dim3((n / 2 + kAggX - 1) / kAggX, (n / 2 + kAggY - 1) / kAggY); }
+
+struct Agg {
+    int I, J, nc, k;  // aggregate, aggregates a row, its first cell
+    bool west, east, south, north;
+    __device__ __forceinline__ explicit Agg(int n) {
+        J = blockIdx.x * kAggX + (threadIdx.x & 31);
+        I = blockIdx.y * kAggY + (threadIdx.x >> 5);
+        nc = n >> 1;
+        k = 2 * I * n + 2 * J;
+        west = J > 0;
+        east = J + 1 < nc;
+        south = I > 0;
+        north = I + 1 < nc;
+    }
+    __device__ __forceinline__ bool inside() const { return I < nc && J < nc; }
+};
+
+// One rounding, whatever the compiler makes of the zeros of absent neighbours.
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+template <class T, int kColour>
+__global__ void __launch_bounds__(kAggX * kAggY) k_gs_agg(Lvl<T> L, bool zero, const CgState* st) {
+    pdl_enter();
+    if (st && st->done) return;
+    const int n = L.n;
+    const Agg A(n);
+    if (!A.inside()) return;
+    const int k0 = A.k, k1 = A.k + n;  // first cells of the two rows
+    if (kColour == 0) {
+        T v0 = L.b[k0], v1 = L.b[k1 + 1];
+        if (!zero) {
+            const T x01 = L.x[k0 + 1], x10 = L.x[k1];
+            const Pair_t<T> n0 = load_pair(L.nf + k0), e1 = load_pair(L.e + k1);
+            const T xe = A.east ? L.x[k1 + 2] : T(0), xw = A.west ? L.x[k0 - 1] : T(0);
+            const T ew = A.west ? L.e[k0 - 1] : T(0), xn = A.north ? L.x[k1 + 1 + n] : T(0);
+            const T ss = A.south ? L.nf[k0 - n] : T(0), xs = A.south ? L.x[k0 - n] : T(0);
+            v0 = mad(L.e[k0], x01, v0);
+            v1 = mad(e1.y, xe, v1);
+            v0 = mad(ew, xw, v0);
+            v1 = mad(e1.x, x10, v1);
+            v0 = mad(n0.x, x10, v0);
+            v1 = mad(L.nf[k1 + 1], xn, v1);
+            v0 = mad(ss, xs, v0);
+            v1 = mad(n0.y, x01, v1);
+        }
+        L.x[k0] = v0 * L.id[k0];
+        L.x[k1 + 1] = v1 * L.id[k1 + 1];
+    } else {
+        const T x00 = L.x[k0], x11 = L.x[k1 + 1];
+        const Pair_t<T> n0 = load_pair(L.nf + k0), e0 = load_pair(L.e + k0);
+        T v0 = L.b[k0 + 1], v1 = L.b[k1];
+        const T xe = A.east ? L.x[k0 + 2] : T(0), xw = A.west ? L.x[k1 - 1] : T(0);
+        const T ew = A.west ? L.e[k1 - 1] : T(0), xn = A.north ? L.x[k1 + n] : T(0);
+        const T ss = A.south ? L.nf[k0 + 1 - n] : T(0), xs = A.south ? L.x[k0 + 1 - n] : T(0);
+        v0 = mad(e0.y, xe, v0);
+        v1 = mad(L.e[k1], x11, v1);
+        v0 = mad(e0.x, x00, v0);
+        v1 = mad(ew, xw, v1);
+        v0 = mad(n0.y, x11, v0);
+        v1 = mad(L.nf[k1], xn, v1);
+        v0 = mad(ss, xs, v0);
+        v1 = mad(n0.x, x00, v1);
+        L.x[k0 + 1] = v0 * L.id[k0 + 1];
+        L.x[k1] = v1 * L.id[k1];
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kAggX * kAggY) k_prolong_gs1_agg(Lvl<T> L, const T* __restrict__ xc,
+                                                                   const CgState* st) {
+    pdl_enter();
+    if (st && st->done) return;
+    const int n = L.n;
+    const Agg A(n);
+    if (!A.inside()) return;
+    const int k0 = A.k, k1 = A.k + n, K = A.I * A.nc + A.J;
+    const T c = xc[K];
+    const T x00 = L.x[k0] + c, x11 = L.x[k1 + 1] + c;
+    const Pair_t<T> n0 = load_pair(L.nf + k0), e0 = load_pair(L.e + k0);
+    T v0 = L.b[k0 + 1], v1 = L.b[k1];
+    const T xe = A.east ? L.x[k0 + 2] + xc[K + 1] : T(0), xw = A.west ? L.x[k1 - 1] + xc[K - 1] : T(0);
+    const T ew = A.west ? L.e[k1 - 1] : T(0), xn = A.north ? L.x[k1 + n] + xc[K + A.nc] : T(0);
+    const T ss = A.south ? L.nf[k0 + 1 - n] : T(0), xs = A.south ? L.x[k0 + 1 - n] + xc[K - A.nc] : T(0);
+    v0 = mad(e0.y, xe, v0);
+    v1 = mad(L.e[k1], x11, v1);
+    v0 = mad(e0.x, x00, v0);
+    v1 = mad(ew, xw, v1);
+    v0 = mad(n0.y, x11, v0);
+    v1 = mad(L.nf[k1], xn, v1);
+    v0 = mad(ss, xs, v0);
+    v1 = mad(n0.x, x00, v1);
+    L.x[k0 + 1] = v0 * L.id[k0 + 1];
+    L.x[k1] = v1 * L.id[k1];
+}
+
+// The 12 neighbourhood values of an aggregate's four cells: x with its ring,
+// and the faces between them (zero outside the domain).
+template <class T>
+struct AggStencil {
+    Pair_t<T> x0, x1, xn, xs, e0, e1, n0, n1, ns;
+    T xw0, xw1, xe0, xe1, ew0, ew1;
+    __device__ __forceinline__ void load(const Agg& A, int n, const T* x, const T* e, const T* nf) {
+        const int k0 = A.k, k1 = A.k + n;
+        Pair_t<T> none;
+        none.x = none.y = T(0);
+        x0 = load_pair(x + k0);
+        x1 = load_pair(x + k1);
+        xn = A.north ? load_pair(x + k1 + n) : none;
+        xs = A.south ? load_pair(x + k0 - n) : none;
+        xw0 = A.west ? x[k0 - 1] : T(0);
+        xw1 = A.west ? x[k1 - 1] : T(0);
+        xe0 = A.east ? x[k0 + 2] : T(0);
+        xe1 = A.east ? x[k1 + 2] : T(0);
+        faces(A, n, e, nf);
+    }
+    __device__ __forceinline__ void faces(const Agg& A, int n, const T* e, const T* nf) {
+        const int k0 = A.k, k1 = A.k + n;
+        Pair_t<T> none;
+        none.x = none.y = T(0);
+        e0 = load_pair(e + k0);
+        e1 = load_pair(e + k1);
+        n0 = load_pair(nf + k0);
+        n1 = load_pair(nf + k1);
+        ns = A.south ? load_pair(nf + k0 - n) : none;
+        ew0 = A.west ? e[k0 - 1] : T(0);
+        ew1 = A.west ? e[k1 - 1] : T(0);
+    }
+};
+
+__global__ void __launch_bounds__(kAggX * kAggY) k_residual_restrict_agg(Lvl<double> L, double* __restrict__ bc,
+                                                                         const CgState* st) {
+    pdl_enter();
+    if (st && st->done) return;
+    const int n = L.n;
+    const Agg A(n);
+    if (!A.inside()) return;
+    AggStencil<double> S;
+    S.load(A, n, L.x, L.e, L.nf);
+    const double2 d0 = load_pair(L.d + A.k), d1 = load_pair(L.d + A.k + n), b0 = load_pair(L.b + A.k),
+                  b1 = load_pair(L.b + A.k + n);
+    auto cell = [](double d, double x, double e, double xe, double w, double xw, double nn, double xn, double s,
+                   double xs) {
+        double v = __dmul_rn(d, x);
+        v = fma(-e, xe, v);
+        v = fma(-w, xw, v);
+        v = fma(-nn, xn, v);
+        return fma(-s, xs, v);
+    };
+    double s = b0.x - cell(d0.x, S.x0.x, S.e0.x, S.x0.y, S.ew0, S.xw0, S.n0.x, S.x1.x, S.ns.x, S.xs.x);
+    s += b0.y - cell(d0.y, S.x0.y, S.e0.y, S.xe0, S.e0.x, S.x0.x, S.n0.y, S.x1.y, S.ns.y, S.xs.y);
+    s += b1.x - cell(d1.x, S.x1.x, S.e1.x, S.x1.y, S.ew1, S.xw1, S.n1.x, S.xn.x, S.n0.x, S.x0.x);
+    s += b1.y - cell(d1.y, S.x1.y, S.e1.y, S.xe1, S.e1.x, S.x1.x, S.n1.y, S.xn.y, S.n0.y, S.x0.y);
+    bc[A.I * A.nc + A.J] = s;
+}
+
+__global__ void __launch_bounds__(kAggX * kAggY)
+    k_residual_restrict_df_agg(Lvl<float> L, const float* __restrict__ elo, const float* __restrict__ nlo,
+                               const float* __restrict__ dlo, const float* __restrict__ blo, float* __restrict__ bc,
+                               const CgState* st) {
+    pdl_enter();
+    if (st && st->done) return;
+    const int n = L.n;
+    const Agg A(n);
+    if (!A.inside()) return;
+    AggStencil<float> H, Q;  // hi parts with x, lo parts
+    H.load(A, n, L.x, L.e, L.nf);
+    Q.faces(A, n, elo, nlo);
+    const int k0 = A.k, k1 = A.k + n;
+    const float2 d0 = load_pair(L.d + k0), d1 = load_pair(L.d + k1), dl0 = load_pair(dlo + k0),
+                 dl1 = load_pair(dlo + k1), b0 = load_pair(L.b + k0), b1 = load_pair(L.b + k1);
+    float2 bl0 = make_float2(0.f, 0.f), bl1 = bl0;
+    if (blo) {
+        bl0 = load_pair(blo + k0);
+        bl1 = load_pair(blo + k1);
+    }
+    DF acc{0.f, 0.f};
+    auto cell = [&](float b, float bl, float d, float dl, float x, float e, float el, float xe, float w, float wl,
+                    float xw, float nn, float nl, float xn, float s, float sl, float xs) {
+        df_add(acc, b, bl);
+        df_axpy(acc, d, dl, x, -1.f);
+        df_axpy(acc, e, el, xe, 1.f);
+        df_axpy(acc, w, wl, xw, 1.f);
+        df_axpy(acc, nn, nl, xn, 1.f);
+        df_axpy(acc, s, sl, xs, 1.f);
+    };
+    cell(b0.x, bl0.x, d0.x, dl0.x, H.x0.x, H.e0.x, Q.e0.x, H.x0.y, H.ew0, Q.ew0, H.xw0, H.n0.x, Q.n0.x, H.x1.x, H.ns.x,
+         Q.ns.x, H.xs.x);
+    cell(b0.y, bl0.y, d0.y, dl0.y, H.x0.y, A.east ? H.e0.y : 0.f, A.east ? Q.e0.y : 0.f, H.xe0, H.e0.x, Q.e0.x, H.x0.x,
+         H.n0.y, Q.n0.y, H.x1.y, H.ns.y, Q.ns.y, H.xs.y);
+    cell(b1.x, bl1.x, d1.x, dl1.x, H.x1.x, H.e1.x, Q.e1.x, H.x1.y, H.ew1, Q.ew1, H.xw1, A.north ? H.n1.x : 0.f,
+         A.north ? Q.n1.x : 0.f, H.xn.x, H.n0.x, Q.n0.x, H.x0.x);
+    cell(b1.y, bl1.y, d1.y, dl1.y, H.x1.y, A.east ? H.e1.y : 0.f, A.east ? Q.e1.y : 0.f, H.xe1, H.e1.x, Q.e1.x, H.x1.x,
+         A.north ? H.n1.y : 0.f, A.north ? Q.n1.y : 0.f, H.xn.y, H.n0.y, Q.n0.y, H.x0.y);
+    bc[A.I * A.nc + A.J] = acc.hi + acc.lo;
+}
+
 // Last post-smoothing pass on level 0 (colour 0) fused with rz = r . z and
 // beta = rz_new / rz (solver.hpp:167-171). z is the level-0 iterate; in the
 // mixed form it is the FP32 iterate widened to FP64 on the fly.
@@ -864,20 +1076,41 @@ void launch_cg_init(const double* f, double h2, int64_t m, double* b, double* r,
 }
 template <class T>
 void launch_gs(const Lvl<T>& L, int colour, bool zero, CgState* st, cudaStream_t s) {
+    if (L.n % 2 == 0) {
+        if (colour == 0)
+            launch_k(k_gs_agg<T, 0>, agg_grid(L.n), kAggX * kAggY, 0, s, L, zero, st);
+        else
+            launch_k(k_gs_agg<T, 1>, agg_grid(L.n), kAggX * kAggY, 0, s, L, false, st);
+        return;
+    }
     launch_k(k_gs<T>, grid_fill(k_gs<T>, colour_count(L.n, colour)), kThreads, 0, s, L, colour, zero, st);
 }
 template <class T>
 void launch_residual_restrict(const Lvl<T>& L, T* bc, CgState* st, cudaStream_t s) {
+    if constexpr (sizeof(T) == 8) {
+        if (L.n % 2 == 0) {
+            launch_k(k_residual_restrict_agg, agg_grid(L.n), kAggX * kAggY, 0, s, L, bc, st);
+            return;
+        }
+    }
     const int64_t nc = (L.n + 1) / 2;
     launch_k(k_residual_restrict<T>, grid_fill(k_residual_restrict<T>, nc * nc), kThreads, 0, s, L, bc, st);
 }
 void launch_residual_restrict_df(const Lvl<float>& L, const float* elo, const float* nlo, const float* dlo,
                                  const float* blo, float* bc, CgState* st, cudaStream_t s) {
+    if (L.n % 2 == 0) {
+        launch_k(k_residual_restrict_df_agg, agg_grid(L.n), kAggX * kAggY, 0, s, L, elo, nlo, dlo, blo, bc, st);
+        return;
+    }
     const int64_t nc = (L.n + 1) / 2;
     launch_k(k_residual_restrict_df, grid_fill(k_residual_restrict_df, nc * nc), kThreads, 0, s, L, elo, nlo, dlo, blo, bc, st);
 }
 template <class T>
 void launch_prolong_gs1(const Lvl<T>& L, const T* xc, CgState* st, cudaStream_t s) {
+    if (L.n % 2 == 0) {
+        launch_k(k_prolong_gs1_agg<T>, agg_grid(L.n), kAggX * kAggY, 0, s, L, xc, st);
+        return;
+    }
     launch_k(k_prolong_gs1<T>, grid_fill(k_prolong_gs1<T>, colour_count(L.n, 1)), kThreads, 0, s, L, xc, st);
 }
 template <class T>
