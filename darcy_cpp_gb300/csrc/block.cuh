@@ -233,6 +233,32 @@ __device__ void block_clear(const BlockViews<T>& V) {
     __syncthreads();
 }
 
+// Cell c of the cycle's copy of a level, in the cycle's precision (FP32 for
+// the mixed form, shared-memory copies for FP64 arrays held on chip), written
+// while the FP64 values are in registers: reading the level back for it took a
+// fifth of the mixed form's setup. (ce, cn): the faces with those on the
+// domain's boundary zero. The FP32 reciprocal diagonal is the correctly
+// rounded reciprocal of the FP32 d (the FP64 id, one FP64 division per cell, is
+// built for FP32 cycles on the coarsest level only); FP64 copies take id as built.
+template <class T>
+__device__ __forceinline__ void block_emit_cell(const Lvl64& H, const PLvl<T>& V, int c, double ce, double cn,
+                                                double dd, double id) {
+    if (!V.e) return;  // not visited
+    if constexpr (sizeof(T) == 4) {
+        ((T*)V.e)[c] = narrow_to<T>(ce);
+        ((T*)V.nf)[c] = narrow_to<T>(cn);
+        const T dk = narrow_to<T>(dd);
+        ((T*)V.d)[c] = dk;
+        // (FP64 zero, tested off the FP64 pipe: a cell outside the domain)
+        ((T*)V.id)[c] = __double_as_longlong(dd) != 0 ? __frcp_rn(dk) : T(0);
+    } else {
+        if (V.e != H.e) ((T*)V.e)[c] = ce;
+        if (V.nf != H.nf) ((T*)V.nf)[c] = cn;
+        if (V.d != H.d) ((T*)V.d)[c] = dd;
+        if (V.id != H.id) ((T*)V.id)[c] = id;
+    }
+}
+
 // The fine level (level.hpp:79-97, validation solver.hpp:68-77) with every
 // face computed once (one division per face instead of two; FP64 division is
 // tens of instructions on the narrow FP64 pipe): the east/north faces and the
@@ -241,12 +267,15 @@ __device__ void block_clear(const BlockViews<T>& V) {
 // east/north face, the same bits since harmonic() is symmetric, so the level
 // equals build_fine's bit for bit. with_id false leaves id unwritten (the
 // FP32 cycle computes its own reciprocal from the FP32 diagonal). `a` has
-// pitch n, the level the padded pitch.
-__device__ __forceinline__ void block_build_fine(const double* __restrict__ a, const Lvl64& L,
-                                                 unsigned long long* bad, bool with_id) {
-    const int n = L.n, np = 2 * ((n + 1) / 2), m = np * np;
+// pitch n, the level the padded pitch; rows by patch_row, an integer division
+// being ~25 instructions a cell.
+template <class T>
+__device__ __forceinline__ void block_build_fine(const double* __restrict__ a, const Lvl64& L, const PLvl<T>& V,
+                                                 unsigned long long* bad, bool with_id, bool emit) {
+    const int n = L.n, nc = V.nc, np = V.np, m = np * np;
+    const unsigned rcp = V.rcp;
     for (int c = threadIdx.x; c < m; c += blockDim.x) {
-        const int i = c / np, j = c - i * np;
+        const int i = patch_row(c >> 1, nc, rcp), j = c - i * np;
         double e = 0.0, nf = 0.0;
         if (i < n && j < n) {
             const int64_t k = (int64_t)i * n + j;
@@ -262,25 +291,30 @@ __device__ __forceinline__ void block_build_fine(const double* __restrict__ a, c
     }
     __syncthreads();
     for (int c = threadIdx.x; c < m; c += blockDim.x) {
-        const int i = c / np, j = c - i * np;
-        double dd = 0.0, id = 0.0;
+        const int i = patch_row(c >> 1, nc, rcp), j = c - i * np;
+        double dd = 0.0, id = 0.0, e = 0.0, nf = 0.0;
         if (i < n && j < n) {
             const double w = (j > 0) ? L.e[c - 1] : L.wb[i];
             const double s = (i > 0) ? L.nf[c - np] : L.sb[j];
-            dd = L.e[c] + w + L.nf[c] + s;
+            e = L.e[c];
+            nf = L.nf[c];
+            dd = e + w + nf + s;
             if (with_id) id = 1.0 / dd;
         }
         L.d[c] = dd;
         if (with_id) L.id[c] = id;
+        if (emit) block_emit_cell<T>(L, V, c, j + 1 < n ? e : 0.0, i + 1 < n ? nf : 0.0, dd, id);
     }
     __syncthreads();
 }
 
 // Galerkin coarse operator (coarsen in setup.cuh) between padded levels.
-__device__ __forceinline__ void block_coarsen(const Lvl64& F, const Lvl64& C, bool with_id) {
-    const int n = F.n, np = 2 * ((n + 1) / 2), nc = C.n, npc = 2 * ((nc + 1) / 2), mc = npc * npc;
+template <class T>
+__device__ __forceinline__ void block_coarsen(const Lvl64& F, const Lvl64& C, const PLvl<T>& V, bool with_id,
+                                              bool emit) {
+    const int n = F.n, np = 2 * ((n + 1) / 2), nc = C.n, npc = V.np, mc = npc * npc;
     for (int c = threadIdx.x; c < mc; c += blockDim.x) {
-        const int I = c / npc, J = c - I * npc;
+        const int I = patch_row(c >> 1, V.nc, V.rcp), J = c - I * npc;
         double ce = 0.0, cw = 0.0, cn = 0.0, cs = 0.0, dd = 0.0, id = 0.0;
         if (I < nc && J < nc) {
             const int i0 = 2 * I, i1 = (2 * I + 1 < n) ? 2 * I + 1 : 2 * I;
@@ -302,6 +336,7 @@ __device__ __forceinline__ void block_coarsen(const Lvl64& F, const Lvl64& C, bo
         C.nf[c] = cn;
         C.d[c] = dd;
         if (with_id) C.id[c] = id;
+        if (emit) block_emit_cell<T>(C, V, c, J + 1 < nc ? ce : 0.0, I + 1 < nc ? cn : 0.0, dd, id);
     }
 }
 
@@ -312,36 +347,6 @@ __device__ __forceinline__ void block_drop_boundary(const Lvl64& L) {
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         L.e[t * np + n - 1] = 0.0;
         L.nf[(n - 1) * np + t] = 0.0;
-    }
-}
-
-// Cycle coefficients of level l in the cycle's precision (FP32 copies for the
-// mixed form, shared-memory copies for FP64 arrays held on chip). The FP32
-// reciprocal diagonal is the correctly rounded reciprocal of the FP32 d (the
-// FP64 id, one FP64 division per cell, is built for FP32 cycles on the
-// coarsest level only); FP64 copies take id as built.
-template <class T>
-__device__ __forceinline__ void block_copy_coeffs(const Lvl64& H, const PLvl<T>& V) {
-    if (!V.e) return;  // not visited
-    const int m = V.np * V.np;
-    if constexpr (sizeof(T) == 4) {
-        for (int k = threadIdx.x; k < m; k += blockDim.x) {
-            ((T*)V.e)[k] = narrow_to<T>(H.e[k]);
-            ((T*)V.nf)[k] = narrow_to<T>(H.nf[k]);
-            const T dk = narrow_to<T>(H.d[k]);
-            ((T*)V.d)[k] = dk;
-            // (FP64 zero, tested off the FP64 pipe: a cell outside the domain)
-            ((T*)V.id)[k] = __double_as_longlong(H.d[k]) != 0 ? __frcp_rn(dk) : T(0);
-        }
-    } else {
-        auto copy = [&](const T* to, const double* from) {
-            if ((const double*)to == from) return;
-            for (int k = threadIdx.x; k < m; k += blockDim.x) ((T*)to)[k] = from[k];
-        };
-        copy(V.e, H.e);
-        copy(V.nf, H.nf);
-        copy(V.d, H.d);
-        copy(V.id, H.id);
     }
 }
 
@@ -366,12 +371,24 @@ __device__ __forceinline__ double2 pair_apply(const Lvl64& L, const double* __re
 }
 
 // y = A x over a block, FP64, returning then(sum x . y).
-template <class F>
+//
+// kAhead: ask for the next pair's lines one step ahead, as the mixed form's
+// other FP64 passes do. Its problems together exceed L2 (4 CTAs an SM hold
+// ~210 MB at 64^2), so a step otherwise starts with a DRAM round trip: 4096 x
+// 64^2 12.9 -> 12.5 ms, 512 x 128^2 18.3 -> 17.6 ms. The FP64 form is bound by the FP64 pipe and
+// measured level (64^2) to 2% slower (128^2): it does not.
+template <bool kAhead, class F>
 __device__ __forceinline__ double block_apply_dot(const Lvl64& L, const double* x, double* y, double* red,
                                                   F&& then) {
     const int n2 = (L.n + 1) / 2, m2 = 2 * n2 * n2;
     double acc = 0.0;
     for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+        if (const int z = q + blockDim.x; kAhead && z < m2) {
+            prefetch_l2(x + 2 * (z + n2));
+            prefetch_l2(L.e + 2 * z);
+            prefetch_l2(L.nf + 2 * z);
+            prefetch_l2(L.d + 2 * z);
+        }
         const double2 xc = reinterpret_cast<const double2*>(x)[q];
         const double2 v = pair_apply(L, x, q, n2, xc);
         reinterpret_cast<double2*>(y)[q] = v;
@@ -418,6 +435,11 @@ __device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V,
             for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
                 const int k = 2 * q + 2 * patch_row(q, nc, L.rcp) * nc;
                 T o0, o1;
+                if (const int z = q + blockDim.x; sizeof(T) == 4 && z < cnt) {
+                    const int kz = 2 * z + 2 * patch_row(z, nc, L.rcp) * nc;
+                    prefetch_l2(r + kz);
+                    prefetch_l2(r + kz + np);
+                }
                 patch_red(L, L.x, L.b, k, o0, o1);
                 L.x[k] = o0;
                 L.x[k + np + 1] = o1;
@@ -443,9 +465,11 @@ __device__ double block_precondition(const BatchArgs& A, const BlockViews<T>& V,
 // columns at once, in the cycle's precision (the FP32 smoothing of the mixed
 // form, with the exact 1 x 1 coarsest solve in FP64), stored row-major; rows
 // and columns of padding cells are zero.
-// Building it in FP64 cost the mixed form about a third of its FP64 work.
+// Building it in FP64 cost the mixed form about a third of its FP64 work. Not
+// inlined: called once a problem, and expanded in the solve it costs the
+// loop there registers (4096 x 64^2 mixed 12.54 -> 12.36 ms).
 template <class T>
-__device__ void block_build_tail(const BatchArgs& A, const BlockViews<T>& V) {
+__device__ __noinline__ void block_build_tail(const BatchArgs& A, const BlockViews<T>& V) {
     const int tl = V.tl, N = V.ntail, pitch = tail_pitch<T>(N);
     const PLvl<T>& L = V.lm[tl];
     const int st = rhs_stride(L.np);
@@ -473,17 +497,24 @@ __device__ unsigned long long block_setup(const BatchArgs& A, const double* a, c
     // FP64 reciprocal diagonals: every level for an FP64 cycle; level 0 for
     // the Jacobi preconditioner; otherwise the coarsest level's exact solve only.
     const bool fp64_id = sizeof(T) == 8 || A.pc != kPcMultigrid;
-    block_build_fine(a, V.h[0], s_bad, fp64_id || V.nlev == 1);
+    const bool mg = A.pc == kPcMultigrid;
+    block_build_fine<T>(a, V.h[0], V.lv[0], s_bad, fp64_id || V.nlev == 1, mg);
     for (int l = 1; l < V.nlev; ++l) {
-        block_coarsen(V.h[l - 1], V.h[l], fp64_id || l == V.nlev - 1);
+        block_coarsen<T>(V.h[l - 1], V.h[l], V.lv[l], fp64_id || l == V.nlev - 1, mg);
         __syncthreads();
         block_drop_boundary(V.h[l - 1]);  // (read by the coarsening just done)
     }
     block_drop_boundary(V.h[V.nlev - 1]);
     __syncthreads();
-    if (A.pc == kPcMultigrid) {
-        for (int l = 0; l < V.nlev; ++l) block_copy_coeffs<T>(V.h[l], V.lv[l]);
-        for (int l = V.tl ? V.tl : V.nlev; l < V.nlev; ++l) block_copy_coeffs<T>(V.h[l], V.lm[l]);
+    if (mg) {
+        if constexpr (sizeof(T) == 4) {  // (FP64: the hierarchy itself)
+            for (int l = V.tl ? V.tl : V.nlev; l < V.nlev; ++l) {
+                const Lvl64& H = V.h[l];
+                const int m = V.lm[l].np * V.lm[l].np;
+                for (int c = threadIdx.x; c < m; c += blockDim.x)
+                    block_emit_cell<T>(H, V.lm[l], c, H.e[c], H.nf[c], H.d[c], 0.0);
+            }
+        }
         __syncthreads();
         if (V.tl && *s_bad == ~0ull) block_build_tail<T>(A, V);
     }

@@ -263,6 +263,9 @@ __device__ __forceinline__ void pdl_enter() {
     pdl_trigger();
 }
 
+// Ask for the line of p in L2 (no effect on shared memory).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.L2 [%0];" ::"l"(p)); }
+
 // ------------------------------------------------------------ reductions
 
 __device__ __forceinline__ double warp_sum(double v) {

@@ -1230,6 +1230,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     const PLvl<T>& L0 = V.lv[0];
     const int np = L0.np, m2 = np * (np / 2);
     const bool mg = A.pc == kPcMultigrid;
+    constexpr bool kAhead = sizeof(T) == 4;  // see block_apply_dot
 
     const unsigned long long bad = block_setup<T>(A, A.a + off, V, s_bad);
     if (bad != ~0ull) {
@@ -1252,14 +1253,20 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     auto rhs = [&](int k) { return (f ? f[k] : A.fscalar) * h2; };  // cell k of the packed arrays
     double* u_out = A.u + off;
 
+    // cells of the domain: f(packed index, padded index)
+    auto for_cells = [&](auto&& fn) {
+        for (int c = threadIdx.x; c < 2 * m2; c += blockDim.x) {
+            const int i = patch_row(c >> 1, L0.nc, L0.rcp), j = c - i * np;
+            if (i < n && j < n) fn(i * n + j, c);
+        }
+    };
     double sb = 0.0;
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-        const int i = k / n, c = i * np + (k - i * n);
+    for_cells([&](int k, int c) {
         const double bk = rhs(k);
         r[c] = bk;
         u[c] = u0 ? u0[k] : 0.0;
         sb += bk * bk;
-    }
+    });
     const double bnorm = block_sum_then(sb, red, [](double t) { return sqrt(t); });
     int iterations = 0, converged = 0;
     bool sound = true;
@@ -1315,11 +1322,10 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         // solution's ||u||_A^2, so a start is kept while the first is below
         // the second. A rejected start costs one more cycle (z = M b).
         if (u0 && A.u0_fallback && !(rz < bu0)) {
-            for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-                const int i = k / n, c = i * np + (k - i * n);
+            for_cells([&](int k, int c) {
                 u[c] = 0.0;
                 r[c] = rhs(k);
-            }
+            });
             residual = 1.0;
             __syncthreads();
             start_cycle();
@@ -1330,6 +1336,10 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         for (int it = 0; it < A.max_iter; ++it) {
             // p = z + beta p (z alone before the first iteration)
             for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+                if (const int z = q + blockDim.x; kAhead && z < m2) {
+                    prefetch_l2(L0.x + 2 * z);
+                    prefetch_l2(p + 2 * z);
+                }
                 const Pair_t<T> zz = load_pair(L0.x + 2 * q);
                 double2 pp = make_double2(widen_f32(zz.x), widen_f32(zz.y));
                 if (it > 0) {
@@ -1341,7 +1351,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             }
             __syncthreads();
             // alpha = rz / (p . Ap), or a breakdown (solver.hpp:149-155)
-            const double alpha = block_apply_dot(h0, p, ap, red, [&](double pap) {
+            const double alpha = block_apply_dot<kAhead>(h0, p, ap, red, [&](double pap) {
                 if (threadIdx.x == 0) s_broke = !(fabs(pap) > 0.0) || !isfinite(pap);
                 return s_rz / pap;
             });
@@ -1353,6 +1363,13 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             }
             double rr = 0.0;
             for (int q = threadIdx.x; q < m2; q += blockDim.x) {
+                if (const int z = q + blockDim.x; kAhead && z < m2) {
+                    prefetch_l2(u + 2 * z);
+                    prefetch_l2(r + 2 * z);
+                    prefetch_l2(p + 2 * z);
+                    prefetch_l2(ap + 2 * z);
+                    prefetch_l2(L0.id + 2 * z);
+                }
                 double2 uu = load_pair(u + 2 * q), rv = load_pair(r + 2 * q);
                 const double2 pp = load_pair(p + 2 * q), av = load_pair(ap + 2 * q);
                 uu.x += alpha * pp.x;
@@ -1388,7 +1405,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     if (A.true_residual) {
         double tr = 0.0;
         for (int q = threadIdx.x; q < m2; q += blockDim.x) {
-            const int i = 2 * q / np, j = 2 * q - i * np;
+            const int i = patch_row(q, L0.nc, L0.rcp), j = 2 * q - i * np;
             const double2 au = pair_apply(h0, u, q, np / 2, load_pair(u + 2 * q));
             if (i < n) {
                 const double r0 = rhs(i * n + j) - au.x;
@@ -1401,10 +1418,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         }
         true_res = block_sum_then(tr, red, [&](double t) { return sqrt(t) / bnorm; });
     }
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-        const int i = k / n;
-        u_out[k] = u[i * np + (k - i * n)];
-    }
+    for_cells([&](int k, int c) { u_out[k] = u[c]; });
     if (threadIdx.x == 0) {
         A.bad[pid] = ~0ull;
         A.iterations[pid] = iterations;

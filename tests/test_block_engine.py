@@ -58,6 +58,18 @@ def test_options_match_the_oracle(darcy, orc, n, options) -> None:
 
 
 @pytest.mark.parametrize("form", ["fp64", "mixed"])
+@pytest.mark.parametrize("options", [{}, {"cycle_index": 1}, {"pre_sweeps": 3, "post_sweeps": 2}])
+@pytest.mark.parametrize("n", [4, 5, 12, 16])
+def test_dense_tails_match_the_oracle(darcy, orc, n, options, form) -> None:
+    """The dense tail from its first level down to side 2, which one thread
+    solves for a column: directly below it, and one or two levels below."""
+    a = field(n, 7)
+    got = darcy.solve_batch(a[None], tol=1e-12, form=form, **options)
+    assert got.all_converged
+    assert rel_l2(got.u[0], orc.solve(a, tol=1e-12, **options)["u"]) < REL_L2
+
+
+@pytest.mark.parametrize("form", ["fp64", "mixed"])
 def test_layout_changes_and_broken_neighbours_leave_no_trace(darcy, form) -> None:
     """Thousands of small problems of two sides, a third of them with a
     non-finite forcing: every CTA meets both sides and broken problems, and
