@@ -92,3 +92,19 @@ def test_layout_changes_and_broken_neighbours_leave_no_trace(darcy, form) -> Non
     for q in (1, 2, 500, 1999, count - 1):
         if q % 3:
             assert rel_l2(got.u[q], want[q % len(fields)]) < REL_L2
+
+
+def test_packed_inputs_reach_their_problems(darcy) -> None:
+    """Fields, forcings and starts of an uneven batch large enough to be packed
+    by several threads (blocks end inside problems): each problem comes out as
+    in a batch of its own, packed by one."""
+    sides = [97, 33, 130, 64, 181, 1, 150, 77] * 6
+    a = [field(n, s) for s, n in enumerate(sides)]
+    rng = np.random.default_rng(3)
+    f = [rng.standard_normal((n, n)) if s % 3 else 2.0 + s for s, n in enumerate(sides)]
+    x0 = [rng.standard_normal((n, n)) * 1e-3 for n in sides]
+    assert sum(x.nbytes for x in a) > 4 << 20
+    got = darcy.solve_batch_uneven(a, f, tol=1e-12, x0=x0)
+    for q in range(0, len(sides), 5):
+        want = darcy.solve_batch_uneven([a[q]], [f[q]], tol=1e-12, x0=[x0[q]])
+        assert rel_l2(got.u[q], want.u[0]) < REL_L2
