@@ -11,19 +11,19 @@
 // The four 32 -> 32 layers carry 97% of the arithmetic. They run as implicit
 // GEMMs on the 5th-generation tensor cores: a CTA takes a tile of 128
 // consecutive pixels (whole image rows when the side is <= 128), stages the
-// input rows it needs in shared memory as three column-shifted copies (dx =
-// -1, 0, +1, zero outside the image), and then every 16-wide K slice of the
-// 128 x 288 im2col matrix (tap (dy, dx), 16 channels) is a plain strided view
-// of one copy, so A needs no im2col pass: one tcgen05.mma (M 128, N 32,
+// input rows it needs in shared memory, zero outside the image, and then every
+// 16-wide K slice of the 128 x 288 im2col matrix (tap (dy, dx), 16 channels) is
+// a plain strided view of them, so A needs no im2col pass: one tcgen05.mma (M 128, N 32,
 // K 16, BF16 in, FP32 accumulate in tensor memory) per slice, 18 per tile,
 // issued by one thread and completed through an mbarrier; tcgen05.ld brings
-// the accumulator back for the epilogue (bias + GELU, or the GELU derivative
-// in the backward pass). The input gradient of a 32 -> 32 layer is the same
+// the accumulator back for the epilogue (bias + GELU, or the product with the
+// GELU's stored slope in the backward pass). The input gradient of a 32 -> 32 layer is the same
 // kernel with the taps flipped and the channel roles of the weights swapped.
 // The 2 -> 32 layer runs the same kernel on an 8-channel padded input, the
 // 32 -> 1 layer with 16 padded output rows. The weight gradients of every
-// layer are tensor-core GEMMs too (k_wgrad_tc: M = (tap, input channel) rows
-// of an im2col staged in shared memory, N = output channels, K = pixels),
+// layer are tensor-core GEMMs too (k_wgrad_tc: M = (tap row, input channel)
+// of three bands staged in shared memory, N = output channels, K = pixels, one
+// accumulator per tap column),
 // written per CTA and summed in a fixed order so training is deterministic.
 // CUDA-core versions of the convolution and of the weight gradients (engine
 // "simt") check the tensor-core ones; the 1 -> 32 input gradient of the
@@ -157,10 +157,13 @@ __device__ __forceinline__ int rc_pixel(const Geom& g, PosRC p) {
 // ------------------------------------------------------------ elementwise
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
+// GELU and, in `slope`, its derivative: one erf for both.
+__device__ __forceinline__ float gelu(float x, float& slope) {
+    const float e = 1.0f + erff(x * 0.70710678118654752f);
+    const float cdf = 0.5f * e;
     const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-    return cdf + x * pdf;
+    slope = cdf + x * pdf;
+    return 0.5f * x * e;
 }
 
 template <class T>
@@ -434,20 +437,43 @@ __global__ void k_gather(const bf16* __restrict__ ds_x, const float* __restrict_
     }
 }
 
+// 32 aligned bytes at once, a whole sector of L2. The convolutions' epilogues
+// hold a pixel's channels in one thread: with 16-byte stores every sector went
+// to L2 twice, half written (a 32 -> 32 layer of 1024 fields of 64 x 64, 257 ->
+// 244 us; the outputs and input gradients of a step on 256 fields 811 -> 695).
+__device__ __forceinline__ void store32(void* p, const uint32_t* w) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+__device__ __forceinline__ void load32(const float* p, float* v) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
 // ---------------------------------------------------- CUDA-core convolution
 //
 // y[p, co] = sum_{tap, ci} x[p + shift(tap), ci] w[co][tap * CIN + ci] with
 // zero padding, FP32 accumulation; one thread per (pixel, output channel); x
 // has XS >= CIN channels per pixel in memory.
-// Epilogue modes: 0 -> pre = y + bias (if pre), act = GELU(y + bias);
-// 1 -> act = y * GELU'(aux) (input gradient through the next GELU);
-// 2 -> outf = y + bias (the linear output layer).
-enum { kEpiGelu = 0, kEpiGeluGrad = 1, kEpiLinear = 2 };
+// Epilogue modes: 0 -> act = GELU(y + bias) and, if `slope`, slope =
+// GELU'(y + bias) for the backward pass; 1 -> act = y * aux (input gradient
+// through a GELU whose slope is aux); 2 -> outf = y + bias (the linear output
+// layer).
+//
+// The slope is kept, in FP32, where the pre-activation used to be: the
+// backward pass took its erf and exp again from it, more arithmetic than the
+// rest of an input gradient. Same values, so the same bits. 256
+// fields of 64 x 64: the four 32 -> 32 layers' outputs and input gradients 938
+// -> 811 us a step; with the slopes asked for ahead of the accumulator and 32
+// bytes at once 654.
+enum { kEpiGelu = 0, kEpiScaled = 1, kEpiLinear = 2 };
 
 template <class TIN, int CIN, int XS = CIN>
 __global__ void k_conv_simt(const TIN* __restrict__ x, const bf16* __restrict__ wB, const float* __restrict__ bias,
                             int cout, int H, int W, int64_t npix, int mode, const float* __restrict__ aux,
-                            float* __restrict__ pre, bf16* __restrict__ act, float* __restrict__ outf) {
+                            float* __restrict__ slope, bf16* __restrict__ act, float* __restrict__ outf) {
     const int64_t total = npix * cout;
     const int hw = H * W;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -467,10 +493,11 @@ __global__ void k_conv_simt(const TIN* __restrict__ x, const bf16* __restrict__ 
         }
         if (mode == kEpiGelu) {
             const float v = acc + bias[co];
-            if (pre) pre[t] = v;
-            act[t] = __float2bfloat16(gelu(v));
-        } else if (mode == kEpiGeluGrad) {
-            act[t] = __float2bfloat16(acc * gelu_grad(aux[t]));
+            float d;
+            act[t] = __float2bfloat16(slope ? gelu(v, d) : gelu(v));
+            if (slope) slope[t] = d;
+        } else if (mode == kEpiScaled) {
+            act[t] = __float2bfloat16(acc * aux[t]);
         } else {
             outf[t] = acc + bias[co];
         }
@@ -478,12 +505,12 @@ __global__ void k_conv_simt(const TIN* __restrict__ x, const bf16* __restrict__ 
 }
 
 // The output layer's input gradient: a 1 -> 32 channel convolution of the FP32
-// dout with the flipped weights wB[co][tap], times GELU'(aux). One thread per
-// (pixel, 8 channels): the nine neighbours are read once for eight outputs and
-// the pre-activations and results move as 16-byte vectors; every output's sum
-// has k_conv_simt's order. Bound by the erf and exp of GELU' (~50 instructions
-// an output): 383 us with one thread an output and its 64-bit divisions, 72
-// us now (256 fields of 64 x 64).
+// dout with the flipped weights wB[co][tap], times the slopes aux. One thread
+// per (pixel, 8 channels): the nine neighbours are read once for eight outputs
+// and the slopes and results move as 16-byte vectors; every output's sum has
+// k_conv_simt's order. 256 fields of 64 x 64: 383 us with one thread an
+// output, its 64-bit divisions and GELU' computed here, 61 us now (205 MB: 30
+// us at the measured copy rate).
 __global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dout, const bf16* __restrict__ wB, int H,
                                                    int W, int64_t npix, const float* __restrict__ aux,
                                                    bf16* __restrict__ act) {
@@ -496,7 +523,8 @@ __global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dou
          p += ((int64_t)gridDim.x * blockDim.x) >> 2) {
         const int64_t img = p < (1ll << 31) ? (int64_t)((unsigned)p / (unsigned)hw) : p / hw;
         const int rem = (int)(p - img * hw), i = rem / W, j = rem - i * W;
-        float acc[8];
+        float acc[8], g[8];
+        load32(aux + p * kC + part * 8, g);
 #pragma unroll
         for (int c = 0; c < 8; ++c) acc[c] = 0.f;
 #pragma unroll
@@ -508,14 +536,10 @@ __global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dou
 #pragma unroll
                 for (int c = 0; c < 8; ++c) acc[c] += v * sw[tap][part * 8 + c];
         }
-        const float4* z = reinterpret_cast<const float4*>(aux + p * kC + part * 8);
-        const float4 z0 = z[0], z1 = z[1];
-        const float g[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
         uint32_t o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const __nv_bfloat162 pr = __floats2bfloat162_rn(acc[2 * e] * gelu_grad(g[2 * e]),
-                                                            acc[2 * e + 1] * gelu_grad(g[2 * e + 1]));
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(acc[2 * e] * g[2 * e], acc[2 * e + 1] * g[2 * e + 1]);
             o[e] = *reinterpret_cast<const uint32_t*>(&pr);
         }
         *reinterpret_cast<uint4*>(act + p * kC + part * 8) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -531,7 +555,7 @@ __global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dou
 // erf of GELU: most of ~1300 instructions a warp and tile; the ALU pipe is
 // 53-60% busy). A 32 -> 32 layer of 1024 fields of 64 x 64: 312 us when a tile
 // was multiplied and written back one after the other, its staging read every
-// sector twice and descriptors were rebuilt for each multiplication; 257 us now.
+// sector twice and descriptors were rebuilt for each multiplication; 240 us now.
 // (Two such groups sharing the weights, one staging buffer each, 32 warps an
 // SM instead of 16: more instructions, 279 us.)
 //
@@ -548,8 +572,8 @@ __global__ void __launch_bounds__(256) k_out_dgrad(const float* __restrict__ dou
 //   CCH = 1: slice j = taps 2j and 2j + 1 (tap 9 does not exist: its B
 //            chunk is zero and its A view repeats tap 8):
 //            start = shift(2j) * 16, LBO = (shift(2j + 1) - shift(2j)) * 16.
-// Epilogues: kEpiGelu (pre-activation FP32 if `pre`, GELU -> BF16 act),
-// kEpiGeluGrad (act = acc * GELU'(aux), BF16), kEpiLinear (outf = acc[0] + b).
+// Epilogues: kEpiGelu (GELU -> BF16 act, its slope FP32 if `slope`),
+// kEpiScaled (act = acc * aux, BF16), kEpiLinear (outf = acc[0] + b).
 constexpr int kConvThreads = 128;
 constexpr int kConvCols = 64;  // tensor-memory columns: two accumulators of 32
 constexpr long long kWaitLimit = 1ll << 24;  // mbarrier polls before a wait is declared lost
@@ -600,10 +624,11 @@ template <int CCH, int NOUT>
 __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict__ x, const bf16* __restrict__ wB,
                                                           const float* __restrict__ bias, Geom g, int64_t ntiles,
                                                           int mode, const float* __restrict__ aux,
-                                                          float* __restrict__ pre, bf16* __restrict__ act,
+                                                          float* __restrict__ slope, bf16* __restrict__ act,
                                                           float* __restrict__ outf, int* __restrict__ err,
                                                           long long first_wait) {
     using S = TcShape<CCH, NOUT>;
+    constexpr bool kScaled = CCH == 4 && NOUT == 32;  // the shape that also computes input gradients
     extern __shared__ __align__(1024) unsigned char sm[];
     const uint32_t stage = tc_stage_bytes(CCH, g.nq);
     unsigned char* sB = sm;
@@ -679,6 +704,13 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict
     __syncwarp();
     stage_next(1);
     for (int i = 0; i < mine; ++i) {
+        const int pix = position_pixel(g, here.s0 + tid);  // row tid of the tile
+        const int64_t p = here.pixel + pix;
+        float z[kScaled ? 32 : 1];  // (asked for ahead of the wait)
+        if (kScaled && mode == kEpiScaled && pix >= 0) {
+#pragma unroll
+            for (int q = 0; q < 32; q += 8) load32(aux + p * kC + q, z + q);
+        }
         // tile i + 1 has landed, tile i is multiplied, every thread has read
         // the accumulator of tile i - 1
         asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -698,13 +730,11 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict
         stage_next(i + 2);  // into the buffer tile i was multiplied from
         float v[32];
         tmem_ld32(tmem + (i & 1) * 32 + ((uint32_t)(warp * 32) << 16), v);
-        const int pix = position_pixel(g, here.s0 + tid);  // row tid of the tile
         if (pix >= 0) {
-            const int64_t p = here.pixel + pix;
-            if (mode == kEpiLinear) {
+            if (NOUT == 16) {  // kEpiLinear
                 outf[p] = v[0] + sBias[0];
             } else {
-                if (mode == kEpiGelu) {
+                if (!kScaled || mode == kEpiGelu) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 4) {
                         const float4 bb = *reinterpret_cast<const float4*>(sBias + c);
@@ -713,35 +743,35 @@ __global__ void __launch_bounds__(kConvThreads) k_conv_tc(const bf16* __restrict
                         v[c + 2] += bb.z;
                         v[c + 3] += bb.w;
                     }
-                    if (pre) {
-                        float4* dst = reinterpret_cast<float4*>(pre + p * kC);
+                    if (slope) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                        for (int q = 0; q < 32; q += 8) {
+                            uint32_t d[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                float sl;
+                                v[q + e] = gelu(v[q + e], sl);
+                                d[e] = __float_as_uint(sl);
+                            }
+                            store32(slope + p * kC + q, d);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) v[c] = gelu(v[c]);
                     }
+                } else {  // kEpiScaled
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) v[c] = gelu(v[c]);
-                } else {  // kEpiGeluGrad
-                    const float4* src = reinterpret_cast<const float4*>(aux + p * kC);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float4 z = src[q];
-                        v[4 * q] *= gelu_grad(z.x);
-                        v[4 * q + 1] *= gelu_grad(z.y);
-                        v[4 * q + 2] *= gelu_grad(z.z);
-                        v[4 * q + 3] *= gelu_grad(z.w);
-                    }
+                    for (int c = 0; c < 32; ++c) v[c] *= z[kScaled ? c : 0];
                 }
-                uint4* dst = reinterpret_cast<uint4*>(act + p * kC);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint32_t w[4];
+                for (int q = 0; q < 32; q += 16) {
+                    uint32_t w[8];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const __nv_bfloat162 pr = __floats2bfloat162_rn(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
+                    for (int e = 0; e < 8; ++e) {
+                        const __nv_bfloat162 pr = __floats2bfloat162_rn(v[q + 2 * e], v[q + 2 * e + 1]);
                         w[e] = *reinterpret_cast<const uint32_t*>(&pr);
                     }
-                    dst[q] = make_uint4(w[0], w[1], w[2], w[3]);
+                    store32(act + p * kC + q, w);
                 }
             }
         }
@@ -1251,7 +1281,7 @@ struct dgpu_net {
     // batch buffers
     int64_t cap = 0, cap_train = 0;  // samples the batch buffers hold
     Buf<bf16> x0, act[5], dpre[2];
-    Buf<float> pre[5], out, target, dout, af, err_e, norm;
+    Buf<float> slope[5], out, target, dout, af, err_e, norm;
     // dataset
     int64_t ds_count = 0;
     Buf<bf16> ds_x;
@@ -1292,7 +1322,7 @@ int net_run(const std::function<void()>& fn) {
     }
 }
 
-// Batch buffers for `count` samples: activations always, pre-activations and
+// Batch buffers for `count` samples: activations always, GELU slopes and
 // gradients only for training.
 void ensure_batch(dgpu_net* N, int64_t count, bool train) {
     const size_t np = (size_t)count * N->hw;
@@ -1303,7 +1333,7 @@ void ensure_batch(dgpu_net* N, int64_t count, bool train) {
         N->cap = count;
     }
     if (train && count > N->cap_train) {
-        for (int l = 0; l < 5; ++l) N->pre[l].ensure(np * kC);
+        for (int l = 0; l < 5; ++l) N->slope[l].ensure(np * kC);
         N->dpre[0].ensure(np * kC);
         N->dpre[1].ensure(np * kC);
         N->target.ensure(np);
@@ -1332,42 +1362,42 @@ const float* bias_of(dgpu_net* N, int l) { return N->w.p + N->T.off_b[l]; }
 
 template <int CCH, int NOUT>
 void launch_tc(dgpu_net* N, int ctas_cap, const bf16* x, const bf16* wB, const float* b, int64_t count, int mode,
-               const float* aux, float* pre, bf16* act, float* outf) {
+               const float* aux, float* slope, bf16* act, float* outf) {
     const int64_t ntiles = count * N->g.tiles_per_img;
     const int ctas = (int)std::min<int64_t>(ntiles, ctas_cap);
     k_conv_tc<CCH, NOUT><<<ctas, kConvThreads, tc_smem_bytes<CCH, NOUT>(N->g.nq), N->stream>>>(
-        x, wB, b, N->g, ntiles, mode, aux, pre, act, outf, N->err.p, N->first_wait);
+        x, wB, b, N->g, ntiles, mode, aux, slope, act, outf, N->err.p, N->first_wait);
     launched(N);
 }
 
 // One 32 -> 32 convolution on the selected engine.
 void conv32(dgpu_net* N, const bf16* x, const bf16* wB, const float* b, int64_t count, int mode, const float* aux,
-            float* pre, bf16* act) {
+            float* slope, bf16* act) {
     const int64_t npix = count * N->hw;
     if (N->engine == DGPU_NET_TENSOR) {
-        launch_tc<4, 32>(N, N->ctas_tc32, x, wB, b, count, mode, aux, pre, act, nullptr);
+        launch_tc<4, 32>(N, N->ctas_tc32, x, wB, b, count, mode, aux, slope, act, nullptr);
     } else {
         k_conv_simt<bf16, 32><<<grid_for(npix * kC, 256, N->sms), 256, 0, N->stream>>>(
-            x, wB, b, kC, N->g.H, N->g.W, npix, mode, aux, pre, act, nullptr);
+            x, wB, b, kC, N->g.H, N->g.W, npix, mode, aux, slope, act, nullptr);
         launched(N);
     }
 }
 
 // Forward pass over `count` samples already in x0. With keep = false the
-// pre-activations are not stored (prediction only).
+// slopes are not stored (prediction only).
 void forward(dgpu_net* N, int64_t count, bool keep) {
     const int64_t npix = count * N->hw;
     if (N->engine == DGPU_NET_TENSOR)
         launch_tc<1, 32>(N, N->ctas_tc_in, N->x0.p, N->wb.p + N->T.off_tc0, bias_of(N, 0), count, kEpiGelu, nullptr,
-                         keep ? N->pre[0].p : nullptr, N->act[0].p, nullptr);
+                         keep ? N->slope[0].p : nullptr, N->act[0].p, nullptr);
     else {
         k_conv_simt<bf16, 2, 8><<<grid_for(npix * kC, 256, N->sms), 256, 0, N->stream>>>(
             N->x0.p, wf(N, 0), bias_of(N, 0), kC, N->g.H, N->g.W, npix, kEpiGelu, nullptr,
-            keep ? N->pre[0].p : nullptr, N->act[0].p, nullptr);
+            keep ? N->slope[0].p : nullptr, N->act[0].p, nullptr);
         launched(N);
     }
     for (int l = 1; l <= 4; ++l)
-        conv32(N, N->act[l - 1].p, wf(N, l), bias_of(N, l), count, kEpiGelu, nullptr, keep ? N->pre[l].p : nullptr,
+        conv32(N, N->act[l - 1].p, wf(N, l), bias_of(N, l), count, kEpiGelu, nullptr, keep ? N->slope[l].p : nullptr,
                N->act[l].p);
     if (N->engine == DGPU_NET_TENSOR)
         launch_tc<4, 16>(N, N->ctas_tc_out, N->act[4].p, N->wb.p + N->T.off_tc5, bias_of(N, 5), count, kEpiLinear,
@@ -1427,12 +1457,12 @@ void backward(dgpu_net* N, int64_t count, float* loss_slot) {
     // the GELU of layer 4 (a 1 -> 32 convolution with the flipped weights)
     wgrad<float, 32, 32, 1>(N, N->act[4].p, N->dout.p, count, 5);
     k_out_dgrad<<<grid_for(npix * 4, 256, N->sms), 256, 0, N->stream>>>(N->dout.p, wt(N, 5), N->g.H, N->g.W, npix,
-                                                                        N->pre[4].p, N->dpre[0].p);
+                                                                        N->slope[4].p, N->dpre[0].p);
     launched(N);
     int cur = 0;  // dpre[cur] holds the gradient at layer l's pre-activation
     for (int l = 4; l >= 1; --l) {
         wgrad<bf16, 32, 32, 32>(N, N->act[l - 1].p, N->dpre[cur].p, count, l);
-        conv32(N, N->dpre[cur].p, wt(N, l), nullptr, count, kEpiGeluGrad, N->pre[l - 1].p, nullptr,
+        conv32(N, N->dpre[cur].p, wt(N, l), nullptr, count, kEpiScaled, N->slope[l - 1].p, nullptr,
                N->dpre[cur ^ 1].p);
         cur ^= 1;
     }
