@@ -928,8 +928,12 @@ __global__ void __launch_bounds__(256) k_reduce_wgrad(const float* __restrict__ 
 // Bound by staging and its waits. With nine shifted copies (36 planes of 128
 // positions, 104 KB a stage, two stages) the kernel took 218 us on 256 fields
 // of 64 x 64; with the bands a stage is 43 KB, four of them are in flight, and
-// it takes 103 us. One CTA an SM, as before: the tiles of one accumulator and
-// their order, and so every gradient's bits, stay what they were.
+// it took 103 us; with a thread's chunk fixed (no loop over planes it skips),
+// lanes along a position's 64 bytes, addresses by addition and a warp of its
+// own to issue the MMAs, 83 us (the output layer's 106 -> 86, the input layer's
+// 71 -> 55). Without staging it would take 50, without the MMAs 81. One CTA an
+// SM, as before: the tiles of one accumulator and their order, and so every
+// gradient's bits, stay what they were.
 template <int CCH, int NOUT>
 struct WgradTc {
     static constexpr int kDataPlanes = 3 * CCH;                         // A planes holding x: plane dy * CCH + chunk
@@ -950,7 +954,8 @@ __host__ __device__ constexpr uint32_t mma_idesc_mn(int M, int N) {
 }
 
 constexpr int kWgSplit = 4;                   // threads per staged position, each with a share of the planes
-constexpr int kWgThreads = kWgSplit * kTile;
+constexpr int kWgStagers = kWgSplit * kTile;
+constexpr int kWgThreads = kWgStagers + 32;   // and a warp that issues the MMAs
 
 // Position q of the bands: `at` = padded position s0 - P - 1 + q as row and
 // column; band dy is dy rows further down.
@@ -959,14 +964,19 @@ __device__ __forceinline__ void wgrad_stage_bands(const bf16* __restrict__ x, co
                                                   uint32_t dst, int share) {
     using W = WgradTc<CCH, 16>;
     const bool in_row = at.c >= 1 && at.c <= g.W;
-    const int pix0 = at.r * g.W + at.c - 1;
+    if constexpr (CCH == 1) {  // one chunk a pixel: thread `share` stages a band
+        if (share >= 3) return;
+        const int r = at.r + share;
+        const bool valid = in_row && r >= 0 && r < g.H;
+        cp_async16(dst + share * W::kAPlane, valid ? x + (pbase + r * g.W + at.c - 1) * 8 : x, valid);
+    } else {  // thread `share` stages its chunk of every band
+        const bf16* src = x + ((pbase + at.r * g.W + at.c - 1) * CCH + share) * 8;
+        const int down = g.W * CCH * 8;
 #pragma unroll
-    for (int pl = 0; pl < 3 * CCH; ++pl) {
-        const int dy = pl / CCH, c = pl - dy * CCH;
-        if ((CCH > 1 ? c : dy) != share) continue;
-        const bool valid = in_row && at.r + dy >= 0 && at.r + dy < g.H;
-        const bf16* src = valid ? x + ((pbase + pix0 + dy * g.W) * CCH + c) * 8 : x;
-        cp_async16(dst + pl * W::kAPlane, src, valid);
+        for (int dy = 0; dy < 3; ++dy) {
+            const bool valid = in_row && at.r + dy >= 0 && at.r + dy < g.H;
+            cp_async16(dst + (dy * CCH + share) * W::kAPlane, valid ? src + dy * down : x, valid);
+        }
     }
 }
 
@@ -974,7 +984,9 @@ template <int CCH, int NOUT, int CIN, int COUT, class TDY>
 __device__ __forceinline__ void wgrad_stage(const bf16* __restrict__ x, const TDY* __restrict__ dy, const Geom& g,
                                             int64_t pbase, int s0, unsigned char* buf) {
     using W = WgradTc<CCH, NOUT>;
-    const int q = threadIdx.x & (kTile - 1), share = threadIdx.x / kTile;
+    // four lanes the 64 contiguous bytes of a position (CCH = 4), or a band each (CCH = 1)
+    const int q = CCH > 1 ? threadIdx.x / kWgSplit : threadIdx.x & (kTile - 1);
+    const int share = CCH > 1 ? threadIdx.x % kWgSplit : threadIdx.x / kTile;
     const uint32_t a = smem_u32(buf);
     const PosRC base = position_rc(g, s0 - g.P - 1 + q);
     wgrad_stage_bands<CCH>(x, g, pbase, base, a + q * 16, share);
@@ -983,11 +995,8 @@ __device__ __forceinline__ void wgrad_stage(const bf16* __restrict__ x, const TD
     const int pix = rc_pixel(g, rc_add(g, base, 1, 1));  // output position s0 + q
     const uint32_t b = a + W::kAPlanes * W::kAPlane;
     if constexpr (sizeof(TDY) == 2) {
-#pragma unroll
-        for (int c = 0; c < W::kBPlanes; ++c) {
-            if (c != share) continue;
-            cp_async16(b + c * W::kBPlane + q * 16, pix >= 0 ? dy + (pbase + pix) * COUT + c * 8 : dy, pix >= 0);
-        }
+        static_assert(W::kBPlanes == kWgSplit, "a plane a thread");
+        cp_async16(b + share * W::kBPlane + q * 16, pix >= 0 ? dy + (pbase + pix) * COUT + share * 8 : dy, pix >= 0);
     } else if (share == 0) {  // one FP32 channel -> BF16 hi in column 0, lo in column 1
         const float d = pix >= 0 ? to_f(dy[pbase + pix]) : 0.f;
         const bf16 hi = __float2bfloat16(d);
@@ -1043,8 +1052,9 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16* __restrict_
     TileWalk ahead(g);
     auto stage = [&](int i) {  // the CTA's next tile, its i-th, into its stage (an empty group past the end)
         if (i < mine) {
-            wgrad_stage<CCH, NOUT, CIN, COUT, TDY>(x, dy, g, ahead.pixel, ahead.s0,
-                                                   sm + (i % W::kStages) * W::kStage);
+            if (tid < kWgStagers)
+                wgrad_stage<CCH, NOUT, CIN, COUT, TDY>(x, dy, g, ahead.pixel, ahead.s0,
+                                                       sm + (i % W::kStages) * W::kStage);
             ahead.step(g);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -1073,7 +1083,7 @@ __global__ void __launch_bounds__(kWgThreads) k_wgrad_tc(const bf16* __restrict_
             failed = true;
             break;
         }
-        if (i < mine && tid == 0) {
+        if (i < mine && tid == kWgStagers) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // MN-major, no swizzle: element (mn, k) at start + (mn / 8) * SBO + (mn % 8) * 2
             // + (k / 8) * LBO + (k % 8) * 16, with SBO = one plane and LBO = 8 positions; the
