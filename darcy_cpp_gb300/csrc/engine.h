@@ -103,7 +103,7 @@ bool programmatic_launch();
 
 // ---- launch wrappers (kernels.cu) ----
 void launch_build_fine(const double* a, const Lvl64& L, unsigned long long* bad, cudaStream_t s);
-void launch_coarsen(const Lvl64& F, const Lvl64& C, cudaStream_t s);
+void launch_coarsen_all(const Lvl64* h, int nlev, cudaStream_t s);
 void launch_to_fp32(const Lvl64& L, float* e, float* nf, float* d, float* id, float* elo, float* nlo, float* dlo,
                     cudaStream_t s);
 

@@ -111,22 +111,52 @@ __device__ __forceinline__ bool grid_sum2_last(double v1, double v2, double* par
 
 // ------------------------------------------------------------- setup kernels
 
-__global__ void k_build_fine(const double* __restrict__ a, Lvl64 L, unsigned long long* bad) {
+constexpr int kChainSide = 32;   // levels of this side and below are built by one CTA
+constexpr int kChainLevels = 8;  // from 2 * kChainSide down to 1
+
+__global__ void __launch_bounds__(kFineX* kFineY)
+    k_build_fine(const double* __restrict__ a, Lvl64 L, unsigned long long* bad) {
     pdl_enter();
-    build_fine<GridScope>(a, L, bad);
+    build_fine(a, L, bad);
 }
 __global__ void k_coarsen(Lvl64 F, Lvl64 C) {
-    pdl_enter(); coarsen<GridScope>(F, C); }
+    pdl_enter();
+    coarsen<GridScope>(F, C);
+}
+
+// The levels of side kChainSide and below in one launch of one CTA: each has a
+// cell a thread at most, and launched on their own they took ~6 us each. With
+// 32-bit row divisions, all levels below 511^2: 67 -> 39 us, 2048^2 235 -> 112.
+struct CoarseChain {
+    Lvl64 h[kChainLevels];  // h[0] built, the others to build
+    int count;
+};
+__global__ void __launch_bounds__(1024) k_coarsen_chain(CoarseChain c) {
+    pdl_enter();
+    for (int l = 1; l < c.count; ++l) {
+        coarsen<BlockScope>(c.h[l - 1], c.h[l]);
+        __syncthreads();
+    }
+}
 __global__ void k_to_fp32(Lvl64 L, float* e, float* nf, float* d, float* id, float* elo, float* nlo, float* dlo) {
     pdl_enter();
     to_fp32<GridScope>(L, e, nf, d, id, elo, nlo, dlo);
 }
 
 void launch_build_fine(const double* a, const Lvl64& L, unsigned long long* bad, cudaStream_t s) {
-    launch_k(k_build_fine, grid_fill(k_build_fine, (int64_t)L.n * L.n), kThreads, 0, s, a, L, bad);
+    const int tiles = ((L.n + kFineX - 1) / kFineX) * ((L.n + kFineY - 1) / kFineY);
+    launch_k(k_build_fine, tiles, kFineX * kFineY, 0, s, a, L, bad);
 }
-void launch_coarsen(const Lvl64& F, const Lvl64& C, cudaStream_t s) {
-    launch_k(k_coarsen, grid_fill(k_coarsen, (int64_t)C.n * C.n), kThreads, 0, s, F, C);
+// Levels 1 .. nlev - 1 from level 0: one launch a level down to side
+// kChainSide, one for the rest.
+void launch_coarsen_all(const Lvl64* h, int nlev, cudaStream_t s) {
+    int l = 1;
+    for (; l < nlev && h[l].n > kChainSide; ++l)
+        launch_k(k_coarsen, grid_fill(k_coarsen, (int64_t)h[l].n * h[l].n), kThreads, 0, s, h[l - 1], h[l]);
+    if (l >= nlev) return;
+    CoarseChain c{};
+    for (c.count = 0; l - 1 + c.count < nlev; ++c.count) c.h[c.count] = h[l - 1 + c.count];
+    launch_k(k_coarsen_chain, 1, 1024, 0, s, c);
 }
 void launch_to_fp32(const Lvl64& L, float* e, float* nf, float* d, float* id, float* elo, float* nlo, float* dlo,
                     cudaStream_t s) {

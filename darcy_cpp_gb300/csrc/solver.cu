@@ -569,7 +569,7 @@ void emit_visit_hybrid(GridPlan& P, int l, bool first, std::vector<int>& cur, cu
 
 void emit_setup(GridPlan& P, cudaStream_t s) {
     launch_build_fine(P.a, P.h[0], &P.st->bad, s);
-    for (int l = 1; l < P.nlev; ++l) launch_coarsen(P.h[l - 1], P.h[l], s);
+    launch_coarsen_all(P.h.data(), P.nlev, s);
     if (P.mixed_mg)
         for (int l = 0; l < P.nlev; ++l)
             launch_to_fp32(P.h[l], (float*)P.lvf[l].e, (float*)P.lvf[l].nf, (float*)P.lvf[l].d,
@@ -1846,7 +1846,7 @@ int64_t dgpu_hierarchy(dgpu_context* ctx, const double* a, int64_t n, double* ou
         CK(cudaMemcpyAsync(bad, &init, 8, cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(da, a, 8 * (size_t)n * n, cudaMemcpyHostToDevice, s));
         launch_build_fine(da, h[0], bad, s);
-        for (size_t l = 1; l < sides.size(); ++l) launch_coarsen(h[l - 1], h[l], s);
+        launch_coarsen_all(h.data(), (int)sides.size(), s);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s));
         int64_t pos = 0;
