@@ -85,6 +85,11 @@ inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Bytes of per-CTA scratch the batched engine needs for a side-n problem.
 size_t block_arena_bytes(int n, bool mixed, size_t smem_budget);
+// The same for a CTA that takes problems of all these sides in turn. Not what
+// the largest side needs: a side just above 8 * 2^k has a smaller dense tail
+// (side 5, 36 columns) than one just below (side 8, 64 columns), and its arena
+// can be the smaller one.
+size_t block_arena_stride(const int* sides, int64_t count, bool mixed, size_t smem_budget);
 int num_levels_for(int n);
 
 // Message returned by dgpu_last_error() on this thread (solver.cu).

@@ -1235,6 +1235,12 @@ size_t block_arena_bytes(int n, bool mixed, size_t sbudget) {
                  : carve<double>(n, nullptr, nullptr, sbudget, nullptr).global_bytes;
 }
 
+size_t block_arena_stride(const int* sides, int64_t count, bool mixed, size_t sbudget) {
+    size_t most = 0;
+    for (int64_t q = 0; q < count; ++q) most = std::max(most, block_arena_bytes(sides[q], mixed, sbudget));
+    return align_up(most);
+}
+
 // One whole PCG solve (solver.hpp:83-174) by one CTA.
 //
 // The loops over cells that need no neighbour walk pairs of horizontally

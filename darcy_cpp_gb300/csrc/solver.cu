@@ -1201,13 +1201,16 @@ void block_solve(dgpu_context* C, int64_t count, const std::vector<int>& sides, 
     CK(cudaMemcpyAsync((void*)A.side, sides.data(), sizeof(int) * count, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync((void*)A.off, off.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
 
+    std::vector<int> distinct = sides;  // what the arenas are sized for
+    std::sort(distinct.begin(), distinct.end());
+    distinct.erase(std::unique(distinct.begin(), distinct.end()), distinct.end());
     // launch with a given shape over `n_prob` entries of `order` from `first`
     // (slot 1: the second compute stream, its own arenas and work counter)
     auto launch = [&](const BlockConfig& cfg, int64_t n_prob, int64_t first = 0, int slot = 0) {
         const int per_sm = mixed ? block_solve_occupancy<float>(cfg.threads, cfg.smem)
                                  : block_solve_occupancy<double>(cfg.threads, cfg.smem);
         const int ctas = (int)std::min<int64_t>(n_prob, (int64_t)C->sms * std::max(per_sm, 1));
-        const size_t stride = align_up(block_arena_bytes(maxside, mixed, cfg.smem));
+        const size_t stride = block_arena_stride(distinct.data(), (int64_t)distinct.size(), mixed, cfg.smem);
         cudaStream_t ls = slot ? C->stream2 : s;
         BatchArgs B = A;
         B.count = (int)n_prob;
