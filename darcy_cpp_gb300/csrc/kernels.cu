@@ -1356,8 +1356,12 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
         // norm; r0 . M r0 (the first preconditioned residual, computed here
         // anyway) estimates the start's ||u - u0||_A^2 and b . u0 the
         // solution's ||u||_A^2, so a start is kept while the first is below
-        // the second. A rejected start costs one more cycle (z = M b).
+        // the second. A rejected start costs one more cycle (z = M b). One that
+        // is not finite, or that overflowed the cycle, has left such values in
+        // every level's iterate and in r's padding, where the next cycle's
+        // passes would read them times a zero face (patch.cuh): clear them.
         if (u0 && A.u0_fallback && !(rz < bu0)) {
+            if (!isfinite(rz) || !isfinite(residual)) block_clear<T>(V);
             for_cells([&](int k, int c) {
                 u[c] = 0.0;
                 r[c] = rhs(k);
