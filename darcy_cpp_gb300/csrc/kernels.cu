@@ -1252,8 +1252,10 @@ size_t block_arena_stride(const int* sides, int64_t count, bool mixed, size_t sb
 // FP64 pipe. On GB300, against the cell-by-cell passes it replaces (256
 // threads, 48 KiB; device time): 4096 x 64^2 mixed 19.6 -> 14.7 ms, FP64 41 ->
 // 31.7 ms, 512 x 128^2 at contrast 1e4 FP64 36 -> 31 ms (512 threads).
-// Returns false when the solve broke down (the arena may hold non-finite
-// values).
+// Returns whether the arena holds finite values only, so that a problem of the
+// same side can take it over: known after a cycle with a finite r . z, to which
+// every cell of every level contributes (an iterate that overflowed, or a tail
+// built from coefficients beyond FP32, makes it infinite or NaN).
 template <class T>
 __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>& V, double* red,
                                 unsigned long long* s_bad) {
@@ -1305,7 +1307,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
     });
     const double bnorm = block_sum_then(sb, red, [](double t) { return sqrt(t); });
     int iterations = 0, converged = 0;
-    bool sound = true;
+    bool sound = false;
     double residual = 0.0;
     if (bnorm == 0.0) {
         for (int k = threadIdx.x; k < n * n; k += blockDim.x) u_out[k] = 0.0;
@@ -1317,7 +1319,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             A.levels[pid] = 1;
             if (A.true_residual) A.true_residual[pid] = 0.0;
         }
-        return true;
+        return false;
     }
 
     double bu0 = 0.0;  // b . u0: estimates the solution's energy ||u||_A^2 = b . u for a close u0
@@ -1372,6 +1374,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
             rz = block_precondition<T>(A, V, red, itself);
         }
         if (threadIdx.x == 0) s_rz = rz;  // r . z of the current direction (thread 0's)
+        sound = isfinite(rz);
         double beta = 0.0;
         for (int it = 0; it < A.max_iter; ++it) {
             // p = z + beta p (z alone before the first iteration)
@@ -1435,6 +1438,7 @@ __device__ bool block_solve_one(const BatchArgs& A, int pid, const BlockViews<T>
                 if (threadIdx.x == 0) s_rz = t;
                 return ratio;
             });
+            sound = isfinite(beta);
         }
     }
 
