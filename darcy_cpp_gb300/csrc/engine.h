@@ -160,6 +160,7 @@ void launch_copy_cast(const double* src, T* dst, int64_t m, cudaStream_t s);
 template <class T>
 void launch_copy_back(const T* src, double* dst, int64_t m, cudaStream_t s);
 
+constexpr size_t kBlockMaxBudget = 200 << 10;  // the largest smem_budget a launch may have
 template <class T>
 void launch_block_solve(const BatchArgs& args, int ctas, int threads, cudaStream_t s);
 template <class T>

@@ -154,8 +154,9 @@ extern "C" int dgpu_random_fields(int64_t n, int64_t count, unsigned long long s
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_amp, amp.data(), sizeof(float) * m, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_C, C.data(), sizeof(float) * m, cudaMemcpyHostToDevice, s);
     const size_t smem = sizeof(float) * 3 * (size_t)m;
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_random_fields, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)  // (the limit belongs to the function, whatever side other threads ask for: the largest need)
+        e = cudaFuncSetAttribute(k_random_fields, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(float) * 3 * kMaxFieldSide * kMaxFieldSide);
     int sms = 0, dev = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

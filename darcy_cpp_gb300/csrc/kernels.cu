@@ -52,6 +52,17 @@ static int grid_fill(void (*kern)(KArgs...), int64_t work, int threads = kThread
     return (int)g;
 }
 
+// Lets launches of a kernel ask for up to `most` bytes of dynamic shared
+// memory. The limit belongs to the function, which every context and thread
+// shares, so it is always set to the most any launch asks for: set to each
+// launch's own need, a smaller one could come between another thread's setting
+// and its launch, which is then refused. On failure the error stays with the
+// runtime, where the caller's check after the launch finds it.
+template <typename... KArgs>
+static bool set_shared_limit(void (*kern)(KArgs...), size_t most) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
+}
+
 // Launches of the grid engine go through launch_k: with programmatic
 // serialization on (set_programmatic_launch), graph edges between them become
 // programmatic so each kernel's launch overlaps its predecessor's tail.
@@ -889,6 +900,7 @@ __global__ void k_copy_back(const T* __restrict__ src, double* __restrict__ dst,
 // itself started after the kernel before it had completed; data written two
 // or more kernels earlier is safe to read before the wait.)
 constexpr int kTailColThreads = 512;
+constexpr size_t kTailColSmem = 224 << 10;  // (side 32, 7 columns: 212 KB)
 
 // Shared-memory layout of the columns kernel: the levels from l0 down.
 // sbase == null: size only.
@@ -1159,7 +1171,7 @@ void launch_tail_columns(const Lvl64* h_dev, const Lvl64* h_host, int l0, int nl
     // one wave of one CTA an SM: 7 columns each for the 1024 columns of side 32
     const int per = std::min(8, (N + 151) / 152);
     const size_t smem = carve_tail(sides.n, l0, nlev, per, nullptr, nullptr);
-    cudaFuncSetAttribute(k_tail_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (!set_shared_limit(k_tail_columns, kTailColSmem)) return;
     launch_k(k_tail_columns, (N + per - 1) / per, kTailColThreads, smem, s, h_dev, sides, l0, nlev, pre, post, gamma,
              top_calls, N, per, Td, Tf);
 }
@@ -1513,15 +1525,15 @@ template <class T>
 int block_solve_occupancy(int threads, size_t smem) {
     // static + dynamic shared memory above 48 KiB needs the opt-in, so set it always
     const size_t bytes = block_smem_bytes(smem, threads);
-    cudaFuncSetAttribute(k_block_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_block_solve<T>, threads, bytes) != cudaSuccess) n = 1;
+    if (!set_shared_limit(k_block_solve<T>, block_smem_bytes(kBlockMaxBudget, 1024)) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_block_solve<T>, threads, bytes) != cudaSuccess) n = 1;
     return n;
 }
 template <class T>
 void launch_block_solve(const BatchArgs& args, int ctas, int threads, cudaStream_t s) {
     const size_t bytes = block_smem_bytes(args.smem_budget, threads);
-    cudaFuncSetAttribute(k_block_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (!set_shared_limit(k_block_solve<T>, block_smem_bytes(kBlockMaxBudget, 1024))) return;
     k_block_solve<T><<<ctas, threads, bytes, s>>>(args);
 }
 

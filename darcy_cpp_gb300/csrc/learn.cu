@@ -1639,7 +1639,9 @@ std::vector<double> unit_solution(int n) {
 template <int CCH, int NOUT>
 int tc_grid(dgpu_net* N, std::string* info) {
     const int smem = tc_smem_bytes<CCH, NOUT>(N->g.nq);
-    NCK(cudaFuncSetAttribute(k_conv_tc<CCH, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // (the limit belongs to the function, not to this network: the largest side's need)
+    NCK(cudaFuncSetAttribute(k_conv_tc<CCH, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)tc_smem_bytes<CCH, NOUT>(make_geom(kMaxSide).nq)));
     NCK(cudaFuncSetAttribute(k_conv_tc<CCH, NOUT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     int api = 0;
     NCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&api, k_conv_tc<CCH, NOUT>, kConvThreads, smem));
@@ -1664,9 +1666,9 @@ int tc_grid(dgpu_net* N, std::string* info) {
 }
 
 template <class TDY, int CIN, int XS, int COUT>
-void set_wgrad_smem(const Geom& g) {
+void set_wgrad_smem() {
     NCK(cudaFuncSetAttribute(k_wgrad<TDY, CIN, XS, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)wgrad_smem(g, CIN, COUT)));
+                             (int)wgrad_smem(make_geom(kMaxSide), CIN, COUT)));
 }
 
 namespace dgpu {
@@ -1779,9 +1781,9 @@ int dgpu_net_create(int side, unsigned long long seed, dgpu_net** out) {
         N->ctas_tc_in = tc_grid<1, 32>(N.get(), &N->info);
         N->ctas_tc_out = tc_grid<4, 16>(N.get(), &N->info);
         N->wg_ctas = N->sms * 4;
-        set_wgrad_smem<float, 32, 32, 1>(N->g);
-        set_wgrad_smem<bf16, 32, 32, 32>(N->g);
-        set_wgrad_smem<bf16, 2, 8, 32>(N->g);
+        set_wgrad_smem<float, 32, 32, 1>();
+        set_wgrad_smem<bf16, 32, 32, 32>();
+        set_wgrad_smem<bf16, 2, 8, 32>();
         N->gpart.ensure((size_t)N->wg_ctas * Wgrad<32, 32>::NV);
         cast_weights(N.get());
         NCK(cudaStreamSynchronize(N->stream));

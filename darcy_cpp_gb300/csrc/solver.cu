@@ -1055,7 +1055,7 @@ void load_tuning(dgpu_context* C) {
         // (a shape the kernel cannot take -- threads not a multiple of 32 in
         // 32..1024, or more shared memory than a CTA has -- is ignored)
         if (std::sscanf(text.c_str() + end + 1, " : [ %d , %llu ]", &threads, &smem) == 2 && threads >= 32 &&
-            threads <= 1024 && threads % 32 == 0 && smem <= 200ull * 1024)
+            threads <= 1024 && threads % 32 == 0 && smem <= kBlockMaxBudget)
             C->tuned[key] = BlockConfigPOD{threads, (size_t)smem};
         pos = end + 1;
     }
