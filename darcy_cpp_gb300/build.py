@@ -89,7 +89,7 @@ def build(verbose: bool = False, force: bool = False) -> tuple[Path, Path]:
     nvcc_version = re.search(r"release ([0-9.]+)", subprocess.run([nvcc, "--version"], capture_output=True,
                                                                    text=True).stdout)
     bind = CSRC / "bindings.cpp"
-    if force or _stale(EXT, [bind, LIB, INCLUDE / "darcy_gpu.h"]):
+    if force or _stale(EXT, [bind, CSRC / "pack.h", LIB, INCLUDE / "darcy_gpu.h"]):
         _run([
             os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
             f"-DDARCY_VERSION=\"{VERSION}\"",

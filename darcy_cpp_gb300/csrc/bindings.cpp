@@ -8,20 +8,19 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
-#include <algorithm>
-#include <atomic>
 #include <cstring>
 #include <memory>
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/darcy_gpu.h"
+#include "pack.h"
 
 namespace py = pybind11;
+using dgpu::pack;
+using dgpu::Piece;
 
 namespace {
 
@@ -124,53 +123,6 @@ std::vector<double> make_x0(const py::object& x0, const std::vector<int64_t>& sh
     if (x0.is_none()) return {};
     const Array arr = x0_array(x0, shape);
     return std::vector<double>(arr.data(), arr.data() + arr.size());
-}
-
-// One stretch of a packed array: `len` numbers copied from src, or `value` where src is null.
-struct Piece {
-    const double* src;
-    double value;
-    size_t len;
-};
-
-// Lay the pieces one after another into dst (call without the GIL). By one
-// thread this is a core's memory bandwidth and the first touch of dst's pages,
-// ~14 GB/s, while the GPU waits: on GB300's Arm host a call with 640 fields of
-// 78 MB took 20.5 ms with one thread, 17.7 with 2, 16.4 with 4, 15.9 with 8
-// and with 16. Below kPackAlone bytes one thread packs: starting the others
-// costs ~50 us (0.77 MB: 1.24 ms a call alone, 1.28 with 8), what they save at
-// ~1 MB.
-constexpr size_t kPackThreads = 8, kPackAlone = size_t(4) << 20, kPackBlock = size_t(1) << 15;
-void pack(const std::vector<Piece>& pieces, double* dst) {
-    std::vector<size_t> at(pieces.size() + 1, 0);  // where each piece begins
-    for (size_t q = 0; q < pieces.size(); ++q) at[q + 1] = at[q] + pieces[q].len;
-    const size_t total = at.back(), blocks = (total + kPackBlock - 1) / kPackBlock;
-    std::atomic<size_t> next{0};
-    auto work = [&]() noexcept {
-        for (size_t b; (b = next.fetch_add(1)) < blocks;) {
-            size_t k = b * kPackBlock;
-            const size_t end = std::min(total, k + kPackBlock);
-            size_t q = (size_t)(std::upper_bound(at.begin(), at.end(), k) - at.begin()) - 1;
-            for (; k < end; ++q) {
-                const size_t n = std::min(at[q + 1], end) - k;
-                if (pieces[q].src)
-                    std::memcpy(dst + k, pieces[q].src + (k - at[q]), n * sizeof(double));
-                else
-                    std::fill_n(dst + k, n, pieces[q].value);
-                k += n;
-            }
-        }
-    };
-    const size_t cores = std::max<size_t>(1, std::thread::hardware_concurrency());
-    const size_t threads = total * sizeof(double) < kPackAlone ? 1 : std::min({kPackThreads, cores, blocks});
-    std::vector<std::thread> helpers;
-    helpers.reserve(threads);
-    try {
-        while (helpers.size() + 1 < threads) helpers.emplace_back(work);
-    } catch (const std::system_error&) {  // no more threads to be had: those there are do the rest
-    }
-    work();
-    for (std::thread& t : helpers) t.join();
 }
 
 py::array_t<double> new_array(std::vector<py::ssize_t> shape) { return py::array_t<double>(shape); }
