@@ -314,12 +314,14 @@ PYBIND11_MODULE(_core, m) {
             double* up = static_cast<double*>(ubig.request().ptr);
             std::vector<double> res((size_t)count);
             std::vector<int> iters((size_t)count), conv((size_t)count), levels((size_t)count);
+            // under the GIL, which other Python threads need to write to the
+            // inputs: the call sees each array as it was at one time
+            pack(pieces, packed.get());
+            if (fpacked) pack(fpieces, fpacked.get());
+            if (u0packed) pack(u0pieces, u0packed.get());
             int rc;
             {
                 py::gil_scoped_release release;
-                pack(pieces, packed.get());
-                if (fpacked) pack(fpieces, fpacked.get());
-                if (u0packed) pack(u0pieces, u0packed.get());
                 rc = dgpu_solve_uneven(context(), count, sides.data(), packed.get(), fpacked.get(), fs, &o,
                                        u0packed.get(), up, iters.data(), res.data(), conv.data(), levels.data());
             }

@@ -17,13 +17,12 @@ struct Piece {
     size_t len;
 };
 
-// Lay the pieces one after another into dst (call without the GIL). By one
-// thread this is a core's memory bandwidth and the first touch of dst's pages,
-// ~14 GB/s, while the GPU waits: on GB300's Arm host a call with 640 fields of
-// 78 MB took 20.5 ms with one thread, 17.7 with 2, 16.4 with 4, 15.9 with 8
-// and with 16. Below kPackAlone bytes one thread packs: starting the others
-// costs ~50 us (0.77 MB: 1.24 ms a call alone, 1.28 with 8), what they save at
-// ~1 MB.
+// Lay the pieces one after another into dst. By one thread this is a core's
+// memory bandwidth and the first touch of dst's pages, ~14 GB/s, while the GPU
+// waits: on GB300's Arm host a call with 640 fields of 78 MB took 20.5 ms with
+// one thread, 17.7 with 2, 16.4 with 4, 15.9 with 8 and with 16. Below
+// kPackAlone bytes one thread packs: starting the others costs ~50 us (0.77 MB:
+// 1.24 ms a call alone, 1.28 with 8), what they save at ~1 MB.
 constexpr size_t kPackThreads = 8, kPackAlone = size_t(4) << 20, kPackBlock = size_t(1) << 15;
 inline void pack(const std::vector<Piece>& pieces, double* dst) {
     std::vector<size_t> at(pieces.size() + 1, 0);  // where each piece begins

@@ -1,0 +1,49 @@
+"""What an uneven batch's call sees of its inputs: each array as it was at one
+time, although other Python threads may write to it."""
+
+from __future__ import annotations
+
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+def test_fields_written_by_another_thread_are_seen_whole() -> None:
+    """A thread rewrites every field, one assignment each (under the GIL), with
+    ones and twos in turn: every problem is the one of ones or the one of twos,
+    whose iterates are half as large (exactly: a power of two), and nothing in
+    between. Tolerance: launch shapes differ, so sums round differently."""
+    import darcy_cpp_gb300 as darcy
+
+    n, count = 256, 200  # 105 MB: packed by several threads
+    ones = np.ones((n, n))
+    u1 = darcy.solve_batch_uneven([ones], max_iter=1).u[0]
+    fields = [ones.copy() for _ in range(count)]
+    views = [memoryview(a).cast("B") for a in fields]
+    values = [ones.tobytes(), (2 * ones).tobytes()]
+    stop = threading.Event()
+
+    def write() -> None:
+        k = 0
+        while not stop.is_set():
+            k += 1
+            for v in views:
+                v[:] = values[k & 1]
+
+    writer = threading.Thread(target=write)
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-4)
+    writer.start()
+    try:
+        for _ in range(6):
+            got = darcy.solve_batch_uneven(fields, max_iter=1)
+            for u in got.u:
+                error = min(np.abs(u - u1).max(), np.abs(u - 0.5 * u1).max())
+                assert error < 1e-10 * np.abs(u1).max()
+    finally:
+        stop.set()
+        writer.join()
+        sys.setswitchinterval(interval)
