@@ -125,6 +125,36 @@ std::vector<double> make_x0(const py::object& x0, const std::vector<int64_t>& sh
     return std::vector<double>(arr.data(), arr.data() + arr.size());
 }
 
+// Arrays and constants laid out one after another (pack.h). Arrays that were
+// converted for this (another type or layout) are packed and let go whenever
+// kConverted bytes of them have come together; the caller's own wait for
+// flush(), so that several threads share the copying.
+class Packed {
+public:
+    void allocate(size_t total) { out_.reset(new double[total]); }
+    void add(const Array& arr, bool converted = false) {
+        keep_.push_back(arr);
+        pieces_.push_back(Piece{arr.data(), 0.0, (size_t)arr.size()});
+        if (converted && (converted_ += (size_t)arr.nbytes()) >= kConverted) flush();
+    }
+    void add(double value, size_t len) { pieces_.push_back(Piece{nullptr, value, len}); }
+    void flush() {
+        pack(pieces_, out_.get() + done_);
+        for (const Piece& p : pieces_) done_ += p.len;
+        pieces_.clear();
+        keep_.clear();
+        converted_ = 0;
+    }
+    const double* data() const { return out_.get(); }  // null if nothing was allocated
+
+private:
+    static constexpr size_t kConverted = size_t(32) << 20;
+    std::unique_ptr<double[]> out_;
+    std::vector<Piece> pieces_;
+    std::vector<Array> keep_;  // what the pieces point into
+    size_t done_ = 0, converted_ = 0;
+};
+
 py::array_t<double> new_array(std::vector<py::ssize_t> shape) { return py::array_t<double>(shape); }
 
 // Per-problem results as numpy arrays (int64 counts, float64 residuals, bool
@@ -269,8 +299,10 @@ PYBIND11_MODULE(_core, m) {
             const dgpu_options o =
                 make_options(tol, max_iter, preconditioner, pre_sweeps, post_sweeps, cycle_index, false, form);
             std::vector<int64_t> sides((size_t)count);
-            std::vector<Piece> pieces, fpieces, u0pieces;
-            std::vector<Array> keep;  // what the pieces point into
+            // Inputs are copied under the GIL, which other Python threads need to
+            // write to them: a call sees each array as it was at one time.
+            Packed packed, fpacked, u0packed;
+            std::vector<Array> keep;
             keep.reserve((size_t)count);
             double fs = 0.0;
             const bool f_list = py::isinstance<py::list>(f) && py::len(f) == (size_t)count && count > 0 &&
@@ -285,45 +317,43 @@ PYBIND11_MODULE(_core, m) {
             for (int64_t q = 0; q < count; ++q) {
                 keep.push_back(py::cast<Array>(fields[q]));
                 auto buf = keep.back().request();
-                const int64_t n = require_square_2d(buf, "each field");
-                sides[q] = n;
-                pieces.push_back(Piece{static_cast<const double*>(buf.ptr), 0.0, (size_t)(n * n)});
-                total += (size_t)(n * n);
+                sides[q] = require_square_2d(buf, "each field");
+                total += (size_t)(sides[q] * sides[q]);
             }
+            packed.allocate(total);
+            if (f_list) fpacked.allocate(total);
+            if (!x0.is_none()) u0packed.allocate(total);
             for (int64_t q = 0; q < count; ++q) {
                 const int64_t n = sides[q];
+                packed.add(keep[(size_t)q]);
                 if (f_list) {
-                    Piece piece{nullptr, 0.0, (size_t)(n * n)};
+                    const py::object fq = py::list(f)[q];
+                    double value;
                     Array arr;
-                    if (rhs_array(py::list(f)[q], n, piece.value, arr)) {
-                        piece.src = arr.data();
-                        keep.push_back(std::move(arr));
-                    }
-                    fpieces.push_back(piece);
+                    if (rhs_array(fq, n, value, arr))
+                        fpacked.add(arr, arr.ptr() != fq.ptr());
+                    else
+                        fpacked.add(value, (size_t)(n * n));
                 }
                 if (!x0.is_none()) {
-                    keep.push_back(x0_array(x0l[q], {n, n}));
-                    u0pieces.push_back(Piece{keep.back().data(), 0.0, (size_t)(n * n)});
+                    const py::object xq = x0l[q];
+                    const Array arr = x0_array(xq, {n, n});
+                    u0packed.add(arr, arr.ptr() != xq.ptr());
                 }
             }
-            std::unique_ptr<double[]> packed(new double[total]), fpacked, u0packed;
-            if (f_list) fpacked.reset(new double[total]);
-            if (!x0.is_none()) u0packed.reset(new double[total]);
+            packed.flush();
+            fpacked.flush();
+            u0packed.flush();
             // the solutions land in one array; each problem's u is a view of it
             py::array_t<double> ubig = new_array({(py::ssize_t)total});
             double* up = static_cast<double*>(ubig.request().ptr);
             std::vector<double> res((size_t)count);
             std::vector<int> iters((size_t)count), conv((size_t)count), levels((size_t)count);
-            // under the GIL, which other Python threads need to write to the
-            // inputs: the call sees each array as it was at one time
-            pack(pieces, packed.get());
-            if (fpacked) pack(fpieces, fpacked.get());
-            if (u0packed) pack(u0pieces, u0packed.get());
             int rc;
             {
                 py::gil_scoped_release release;
-                rc = dgpu_solve_uneven(context(), count, sides.data(), packed.get(), fpacked.get(), fs, &o,
-                                       u0packed.get(), up, iters.data(), res.data(), conv.data(), levels.data());
+                rc = dgpu_solve_uneven(context(), count, sides.data(), packed.data(), fpacked.data(), fs, &o,
+                                       u0packed.data(), up, iters.data(), res.data(), conv.data(), levels.data());
             }
             check(rc);
             py::list us;

@@ -1,13 +1,40 @@
-"""What an uneven batch's call sees of its inputs: each array as it was at one
-time, although other Python threads may write to it."""
+"""What an uneven batch's call sees of its inputs, and holds of them: each array
+as it was at one time, although other Python threads may write to it, and no
+more than a bounded amount of converted copies."""
 
 from __future__ import annotations
 
 import sys
 import threading
+import tracemalloc
 
 import numpy as np
 import pytest
+
+N, COUNT = 256, 200  # 0.5 MB an array in FP64, 105 MB together
+
+
+def peak_of_call(forcing) -> int:
+    import darcy_cpp_gb300 as darcy
+
+    fields = [np.full((N, N), 2.0)] * COUNT
+    tracemalloc.start()
+    try:
+        darcy.solve_batch_uneven(fields, forcing, max_iter=1, x0=forcing)
+    except RuntimeError:  # no GPU here: the inputs have been packed by then
+        pass
+    peak = tracemalloc.get_traced_memory()[1]
+    tracemalloc.stop()
+    return peak
+
+
+def test_converted_forcings_and_starts_are_not_all_held_at_once() -> None:
+    """FP32 forcings and starts need FP64 copies, 210 MB of them. Beyond what
+    the call with FP64 arrays (no copies) traces, the solutions included, at
+    most two bounded sets of 32 MB and an array each may be alive."""
+    plain = peak_of_call([np.ones((N, N))] * COUNT)
+    converted = peak_of_call([np.ones((N, N), dtype=np.float32)] * COUNT)
+    assert converted - plain < (72 << 20)
 
 
 @pytest.mark.gpu
