@@ -305,20 +305,35 @@ __global__ void k_prolong_gs1(Lvl<T> L, const T* xc, const CgState* st) {
 // (their rows have no aligned pairs): the same bits. Bound by HBM (FP32) and
 // the FP64 pipe. us a launch on GB300 at 2048^2, one cell a thread -> here:
 //                               FP64           FP32
-//   red, zero start          10.7 ->  9.6    6.7 ->  5.4
-//   black                    32.6 -> 32.2   11.0 ->  8.2
-//   residual + restriction   59.3 -> 51.6   34.5 -> 24.3  (double-float)
-//   prolongation + black     40.9 -> 36.1   16.0 ->  9.6
-// An even side always takes these: at every size measured (64 up) none is slower.
-constexpr int kAggX = 32, kAggY = 8;  // aggregates a CTA covers
-static dim3 agg_grid(int n) { return dim3((n / 2 + kAggX - 1) / kAggX, (n / 2 + kAggY - 1) / kAggY); }
+//   red, zero start          10.4 ->  9.1    6.3 ->  5.3
+//   black                    32.1 -> 31.2   10.9 ->  8.2
+//   residual + restriction   59.0 -> 52.2   34.1 -> 24.0  (double-float)
+//   prolongation + black     40.6 -> 33.2   15.7 ->  9.1
+// A CTA covers 32 x 4 aggregates in FP64 and 32 x 8 in FP32. FP64: with 8 rows
+// a level of side 200 to 700 is 1.2 to 3.2 CTAs an SM, and the SMs that hold
+// one more than the others finish last: solves with two sweeps a side, which
+// run these at every level, took up to 7% longer than with one cell a thread.
+// ms a solve, one cell a thread -> 8 rows -> 4 rows: 300^2 8.6, 9.0, 8.7; 400^2
+// 9.8, 10.4, 9.9; 700^2 20.5, 21.9, 20.6; 1200^2 45.3, 46.7, 44.6. (Two rows or
+// one, also for small levels only: slower at 150 to 700.) FP32: at 4 rows the
+// launch of the CTAs shows (red at 2048^2 8.7 us).
+constexpr int kAggX = 32;
+template <class T>
+constexpr int kAggY = sizeof(T) == 8 ? 4 : 8;
+template <class T>
+constexpr int kAggThreads = kAggX * kAggY<T>;
+template <class T>
+static dim3 agg_grid(int n) {
+    return dim3((n / 2 + kAggX - 1) / kAggX, (n / 2 + kAggY<T> - 1) / kAggY<T>);
+}
 
+template <class T>
 struct Agg {
     int I, J, nc, k;  // aggregate, aggregates a row, its first cell
     bool west, east, south, north;
     __device__ __forceinline__ explicit Agg(int n) {
         J = blockIdx.x * kAggX + (threadIdx.x & 31);
-        I = blockIdx.y * kAggY + (threadIdx.x >> 5);
+        I = blockIdx.y * kAggY<T> + (threadIdx.x >> 5);
         nc = n >> 1;
         k = 2 * I * n + 2 * J;
         west = J > 0;
@@ -334,11 +349,11 @@ __device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_
 __device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 template <class T, int kColour>
-__global__ void __launch_bounds__(kAggX * kAggY) k_gs_agg(Lvl<T> L, bool zero, const CgState* st) {
+__global__ void __launch_bounds__(kAggThreads<T>) k_gs_agg(Lvl<T> L, bool zero, const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
     const int n = L.n;
-    const Agg A(n);
+    const Agg<T> A(n);
     if (!A.inside()) return;
     const int k0 = A.k, k1 = A.k + n;  // first cells of the two rows
     if (kColour == 0) {
@@ -381,12 +396,12 @@ __global__ void __launch_bounds__(kAggX * kAggY) k_gs_agg(Lvl<T> L, bool zero, c
 }
 
 template <class T>
-__global__ void __launch_bounds__(kAggX * kAggY) k_prolong_gs1_agg(Lvl<T> L, const T* __restrict__ xc,
-                                                                   const CgState* st) {
+__global__ void __launch_bounds__(kAggThreads<T>) k_prolong_gs1_agg(Lvl<T> L, const T* __restrict__ xc,
+                                                                     const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
     const int n = L.n;
-    const Agg A(n);
+    const Agg<T> A(n);
     if (!A.inside()) return;
     const int k0 = A.k, k1 = A.k + n, K = A.I * A.nc + A.J;
     const T c = xc[K];
@@ -414,7 +429,7 @@ template <class T>
 struct AggStencil {
     Pair_t<T> x0, x1, xn, xs, e0, e1, n0, n1, ns;
     T xw0, xw1, xe0, xe1, ew0, ew1;
-    __device__ __forceinline__ void load(const Agg& A, int n, const T* x, const T* e, const T* nf) {
+    __device__ __forceinline__ void load(const Agg<T>& A, int n, const T* x, const T* e, const T* nf) {
         const int k0 = A.k, k1 = A.k + n;
         Pair_t<T> none;
         none.x = none.y = T(0);
@@ -428,7 +443,7 @@ struct AggStencil {
         xe1 = A.east ? x[k1 + 2] : T(0);
         faces(A, n, e, nf);
     }
-    __device__ __forceinline__ void faces(const Agg& A, int n, const T* e, const T* nf) {
+    __device__ __forceinline__ void faces(const Agg<T>& A, int n, const T* e, const T* nf) {
         const int k0 = A.k, k1 = A.k + n;
         Pair_t<T> none;
         none.x = none.y = T(0);
@@ -442,12 +457,12 @@ struct AggStencil {
     }
 };
 
-__global__ void __launch_bounds__(kAggX * kAggY) k_residual_restrict_agg(Lvl<double> L, double* __restrict__ bc,
-                                                                         const CgState* st) {
+__global__ void __launch_bounds__(kAggThreads<double>)
+    k_residual_restrict_agg(Lvl<double> L, double* __restrict__ bc, const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
     const int n = L.n;
-    const Agg A(n);
+    const Agg<double> A(n);
     if (!A.inside()) return;
     AggStencil<double> S;
     S.load(A, n, L.x, L.e, L.nf);
@@ -468,14 +483,14 @@ __global__ void __launch_bounds__(kAggX * kAggY) k_residual_restrict_agg(Lvl<dou
     bc[A.I * A.nc + A.J] = s;
 }
 
-__global__ void __launch_bounds__(kAggX * kAggY)
+__global__ void __launch_bounds__(kAggThreads<float>)
     k_residual_restrict_df_agg(Lvl<float> L, const float* __restrict__ elo, const float* __restrict__ nlo,
                                const float* __restrict__ dlo, const float* __restrict__ blo, float* __restrict__ bc,
                                const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
     const int n = L.n;
-    const Agg A(n);
+    const Agg<float> A(n);
     if (!A.inside()) return;
     AggStencil<float> H, Q;  // hi parts with x, lo parts
     H.load(A, n, L.x, L.e, L.nf);
@@ -1120,9 +1135,9 @@ template <class T>
 void launch_gs(const Lvl<T>& L, int colour, bool zero, CgState* st, cudaStream_t s) {
     if (L.n % 2 == 0) {
         if (colour == 0)
-            launch_k(k_gs_agg<T, 0>, agg_grid(L.n), kAggX * kAggY, 0, s, L, zero, st);
+            launch_k(k_gs_agg<T, 0>, agg_grid<T>(L.n), kAggThreads<T>, 0, s, L, zero, st);
         else
-            launch_k(k_gs_agg<T, 1>, agg_grid(L.n), kAggX * kAggY, 0, s, L, false, st);
+            launch_k(k_gs_agg<T, 1>, agg_grid<T>(L.n), kAggThreads<T>, 0, s, L, false, st);
         return;
     }
     launch_k(k_gs<T>, grid_fill(k_gs<T>, colour_count(L.n, colour)), kThreads, 0, s, L, colour, zero, st);
@@ -1131,7 +1146,7 @@ template <class T>
 void launch_residual_restrict(const Lvl<T>& L, T* bc, CgState* st, cudaStream_t s) {
     if constexpr (sizeof(T) == 8) {
         if (L.n % 2 == 0) {
-            launch_k(k_residual_restrict_agg, agg_grid(L.n), kAggX * kAggY, 0, s, L, bc, st);
+            launch_k(k_residual_restrict_agg, agg_grid<T>(L.n), kAggThreads<T>, 0, s, L, bc, st);
             return;
         }
     }
@@ -1141,7 +1156,7 @@ void launch_residual_restrict(const Lvl<T>& L, T* bc, CgState* st, cudaStream_t 
 void launch_residual_restrict_df(const Lvl<float>& L, const float* elo, const float* nlo, const float* dlo,
                                  const float* blo, float* bc, CgState* st, cudaStream_t s) {
     if (L.n % 2 == 0) {
-        launch_k(k_residual_restrict_df_agg, agg_grid(L.n), kAggX * kAggY, 0, s, L, elo, nlo, dlo, blo, bc, st);
+        launch_k(k_residual_restrict_df_agg, agg_grid<float>(L.n), kAggThreads<float>, 0, s, L, elo, nlo, dlo, blo, bc, st);
         return;
     }
     const int64_t nc = (L.n + 1) / 2;
@@ -1150,7 +1165,7 @@ void launch_residual_restrict_df(const Lvl<float>& L, const float* elo, const fl
 template <class T>
 void launch_prolong_gs1(const Lvl<T>& L, const T* xc, CgState* st, cudaStream_t s) {
     if (L.n % 2 == 0) {
-        launch_k(k_prolong_gs1_agg<T>, agg_grid(L.n), kAggX * kAggY, 0, s, L, xc, st);
+        launch_k(k_prolong_gs1_agg<T>, agg_grid<T>(L.n), kAggThreads<T>, 0, s, L, xc, st);
         return;
     }
     launch_k(k_prolong_gs1<T>, grid_fill(k_prolong_gs1<T>, colour_count(L.n, 1)), kThreads, 0, s, L, xc, st);
