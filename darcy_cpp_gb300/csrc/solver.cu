@@ -227,6 +227,7 @@ struct GridPlan {
 struct BlockConfigPOD {
     int threads;
     size_t smem;
+    bool pinned;  // by the user's own file, not timed by the tuner
 };
 
 }  // namespace
@@ -1034,10 +1035,18 @@ std::string tune_file() {
     return "autotune.json";
 }
 
-// The cache file is one JSON object: {"<device>|<key>": [threads, smem], ...}.
+// The cache file is one JSON object: {"<device>|<key>": [threads, smem, version],
+// ...}. The version is that of the kernel the shape was timed with: raised
+// whenever k_block_solve or its arena's layout change so that another shape may
+// win, and entries of other versions are timed again. In a file named by
+// DARCY_GPU_TUNE_FILE an entry without a version is a shape its owner pins;
+// the default file is the tuner's own, and one without is from before versions.
+constexpr int kShapeVersion = 2;
+
 void load_tuning(dgpu_context* C) {
     if (C->tune_loaded) return;
     C->tune_loaded = true;
+    const bool own = std::getenv("DARCY_GPU_TUNE_FILE") == nullptr;
     FILE* fp = std::fopen(tune_file().c_str(), "r");
     if (!fp) return;
     std::string text;
@@ -1050,13 +1059,14 @@ void load_tuning(dgpu_context* C) {
         const size_t end = text.find('"', pos + 1);
         if (end == std::string::npos) break;
         const std::string key = text.substr(pos + 1, end - pos - 1);
-        int threads = 0;
+        int threads = 0, version = 0;
         unsigned long long smem = 0;
         // (a shape the kernel cannot take -- threads not a multiple of 32 in
         // 32..1024, or more shared memory than a CTA has -- is ignored)
-        if (std::sscanf(text.c_str() + end + 1, " : [ %d , %llu ]", &threads, &smem) == 2 && threads >= 32 &&
-            threads <= 1024 && threads % 32 == 0 && smem <= kBlockMaxBudget)
-            C->tuned[key] = BlockConfigPOD{threads, (size_t)smem};
+        const int read = std::sscanf(text.c_str() + end + 1, " : [ %d , %llu , %d", &threads, &smem, &version);
+        if ((read == 3 ? version == kShapeVersion : read == 2 && !own) && threads >= 32 && threads <= 1024 &&
+            threads % 32 == 0 && smem <= kBlockMaxBudget)
+            C->tuned[key] = BlockConfigPOD{threads, (size_t)smem, read == 2};
         pos = end + 1;
     }
 }
@@ -1073,9 +1083,11 @@ void save_tuning(dgpu_context* C) {
     if (!fp) return;
     std::fprintf(fp, "{\n");
     size_t q = 0;
-    for (const auto& kv : C->tuned)
-        std::fprintf(fp, "  \"%s\": [%d, %zu]%s\n", kv.first.c_str(), kv.second.threads, kv.second.smem,
-                     ++q < C->tuned.size() ? "," : "");
+    for (const auto& kv : C->tuned) {
+        std::fprintf(fp, "  \"%s\": [%d, %zu", kv.first.c_str(), kv.second.threads, kv.second.smem);
+        if (!kv.second.pinned) std::fprintf(fp, ", %d", kShapeVersion);
+        std::fprintf(fp, "]%s\n", ++q < C->tuned.size() ? "," : "");
+    }
     std::fprintf(fp, "}\n");
     std::fclose(fp);
 }
@@ -1328,7 +1340,7 @@ void block_solve(dgpu_context* C, int64_t count, const std::vector<int>& sides, 
                 }
             }
         }
-        C->tuned[key] = BlockConfigPOD{cfg.threads, cfg.smem};
+        C->tuned[key] = BlockConfigPOD{cfg.threads, cfg.smem, false};
         save_tuning(C);
     }
     C->last_block_threads = cfg.threads;
