@@ -128,6 +128,7 @@ void launch_gs0_dot(const Lvl<T>& L, const double* r, CgState* st, double* parti
 // Dense coarse-tail operator: columns (setup) and application (per visit).
 void launch_tail_columns(const Lvl64* h_dev, const Lvl64* h_host, int l0, int nlev, int pre, int post, int gamma,
                          int top_calls, int N, double* Td, float* Tf, cudaStream_t s);
+int tail_columns_per_cta(const int* sides, int l0, int nlev, int N, int sms);  // columns a CTA builds
 template <class T>
 void launch_tail_matvec(const T* M, int N, const T* b, T* x, CgState* st, cudaStream_t s);
 // Fused level visits (pre_sweeps = post_sweeps = 1): tile-staged red+black

@@ -1179,12 +1179,21 @@ void launch_gs0_dot(const Lvl<T>& L, const double* r, CgState* st, double* parti
         launch_k(k_gs0_dot<T, false>, grid_fill(k_gs0_dot<T, false>, colour_count(L.n, 0)), kThreads, 0, s, L, r, st,
                  partials);
 }
+// One wave of one CTA an SM where eight columns are enough for that and their
+// vectors fit: 7 columns each for the 1024 columns of side 32 on 152 SMs.
+int tail_columns_per_cta(const int* sides, int l0, int nlev, int N, int sms) {
+    int per = std::min(8, (N + sms - 1) / sms);
+    while (per > 1 && carve_tail(sides, l0, nlev, per, nullptr, nullptr) > kTailColSmem) --per;
+    return per;
+}
 void launch_tail_columns(const Lvl64* h_dev, const Lvl64* h_host, int l0, int nlev, int pre, int post, int gamma,
                          int top_calls, int N, double* Td, float* Tf, cudaStream_t s) {
     TailSides sides{};
     for (int l = 0; l < nlev; ++l) sides.n[l] = h_host[l].n;
-    // one wave of one CTA an SM: 7 columns each for the 1024 columns of side 32
-    const int per = std::min(8, (N + 151) / 152);
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int per = tail_columns_per_cta(sides.n, l0, nlev, N, std::max(sms, 1));
     const size_t smem = carve_tail(sides.n, l0, nlev, per, nullptr, nullptr);
     if (!set_shared_limit(k_tail_columns, kTailColSmem)) return;
     launch_k(k_tail_columns, (N + per - 1) / per, kTailColThreads, smem, s, h_dev, sides, l0, nlev, pre, post, gamma,
