@@ -42,14 +42,10 @@ __device__ __forceinline__ double apply_cell(const Lvl64& L, const double* __res
 // one column per unit right-hand side, all columns at once) and the cycle
 // applies it with one product per visit of level tl - 1 instead of visiting
 // 2^k levels below. Same operator as the recursion, to rounding.
-// Shared by host sizing and device carving (gbase/sbase == null: size only).
+// Shared by host sizing and device carving (gbase/sbase == null: size only);
+// returns the arena's bytes.
 constexpr int kBlockTailSide = 8;
 constexpr int kBlockLevels = 20;  // sides below 2^17: more than the int cell index allows
-
-struct BlockLayout {
-    size_t global_bytes, smem_bytes;
-    int nlev;
-};
 
 template <class T>
 struct BlockViews {
@@ -63,7 +59,7 @@ struct BlockViews {
 };
 
 template <class T>
-__host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sbudget, BlockViews<T>* v) {
+__host__ __device__ size_t carve(int n, char* gbase, char* sbase, size_t sbudget, BlockViews<T>* v) {
     size_t goff = 0, soff = 0;
     // `lead` and `trail` bytes of guard around an array of `bytes` (multiples of 16)
     auto gtake = [&](size_t lead, size_t bytes, size_t trail) -> char* {
@@ -189,7 +185,7 @@ __host__ __device__ BlockLayout carve(int n, char* gbase, char* sbase, size_t sb
             if (v) v->lm[l] = M;
         }
     }
-    return BlockLayout{goff, soff, nlev};
+    return goff;
 }
 
 // Zeroes what the stencils may read before a pass has written it: the guards

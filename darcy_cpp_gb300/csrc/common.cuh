@@ -176,11 +176,11 @@ __device__ __forceinline__ T narrow_to(double x) {
 
 // Red-black Gauss-Seidel, one colour, in place (level.hpp:145-161).
 // `zero` means x is known to be 0: the update collapses to x = b / d.
-template <class S, class T>
+template <class T>
 __device__ __forceinline__ void gs_colour(const Lvl<T> L, int c, bool zero) {
     const int n = L.n;
     const int64_t cnt = colour_count(n, c);
-    for (int64_t t = S::start(); t < cnt; t += S::stride()) {
+    for (int64_t t = GridScope::start(); t < cnt; t += GridScope::stride()) {
         int i, j;
         colour_cell(n, c, t, i, j);
         const int64_t k = (int64_t)i * n + j;
@@ -211,11 +211,11 @@ __device__ __forceinline__ T cell_residual(const Lvl<T>& L, int i, int j) {
 // Fused residual + restriction: b_c = P^T (b - A x), summed over each 2x2
 // aggregate in the reference order (level.hpp:214-227). The coarse iterate is
 // not zero-filled here: the first coarse smoothing pass runs in `zero` mode.
-template <class S, class T>
+template <class T>
 __device__ __forceinline__ void residual_restrict(const Lvl<T> L, T* bc) {
     const int n = L.n, nc = (n + 1) / 2;
     const int64_t mc = (int64_t)nc * nc;
-    for (int64_t K = S::start(); K < mc; K += S::stride()) {
+    for (int64_t K = GridScope::start(); K < mc; K += GridScope::stride()) {
         const int I = (int)(K / nc), J = (int)(K - (int64_t)I * nc);
         const int i0 = 2 * I, i1 = (2 * I + 1 < n) ? 2 * I + 1 : 2 * I;
         const int j0 = 2 * J, j1 = (2 * J + 1 < n) ? 2 * J + 1 : 2 * J;
@@ -231,11 +231,11 @@ __device__ __forceinline__ void residual_restrict(const Lvl<T> L, T* bc) {
 // and the colour-0 pass that follows overwrites every colour-0 cell, so the
 // injected correction only has to be seen through the neighbours here:
 // exactly the values level.hpp:230-237 followed by :145-161 would use.
-template <class S, class T>
+template <class T>
 __device__ __forceinline__ void prolong_gs1(const Lvl<T> L, const T* xc) {
     const int n = L.n, nc = (n + 1) / 2;
     const int64_t cnt = colour_count(n, 1);
-    for (int64_t t = S::start(); t < cnt; t += S::stride()) {
+    for (int64_t t = GridScope::start(); t < cnt; t += GridScope::stride()) {
         int i, j;
         colour_cell(n, 1, t, i, j);
         const int64_t k = (int64_t)i * n + j;

@@ -1,11 +1,14 @@
 // sm_103a kernels of the darcy GB300 engine.
 //
-// Two engines share the level operations of common.cuh:
+// Two engines:
 //   * the grid engine (one solve spread over the whole GPU): one kernel per
-//     phase on the large levels, the coarse tail handed to one CTA, the PCG
-//     scalars kept on the device so that no iteration waits for the host;
-//   * the block engine (batched solves): one CTA runs a whole PCG solve of one
-//     problem, pulling problems from a work counter, largest first.
+//     phase on the large levels (common.cuh, and by 2 x 2 aggregates below), one
+//     per visit on the middle ones (fused.cuh), a dense operator for the levels
+//     of side 32 and less, the PCG scalars kept on the device so that no
+//     iteration waits for the host;
+//   * the block engine (batched solves, block.cuh and patch.cuh): one CTA runs a
+//     whole PCG solve of one problem, pulling problems from a work counter,
+//     largest first.
 #include <math.h>
 
 #include <cstdlib>
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(1024) k_coarsen_chain(CoarseChain c) {
 }
 __global__ void k_to_fp32(Lvl64 L, float* e, float* nf, float* d, float* id, float* elo, float* nlo, float* dlo) {
     pdl_enter();
-    to_fp32<GridScope>(L, e, nf, d, id, elo, nlo, dlo);
+    to_fp32(L, e, nf, d, id, elo, nlo, dlo);
 }
 
 void launch_build_fine(const double* a, const Lvl64& L, unsigned long long* bad, cudaStream_t s) {
@@ -241,13 +244,13 @@ template <class T>
 __global__ void k_gs(Lvl<T> L, int c, bool zero, const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
-    gs_colour<GridScope>(L, c, zero);
+    gs_colour(L, c, zero);
 }
 template <class T>
 __global__ void k_residual_restrict(Lvl<T> L, T* bc, const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
-    residual_restrict<GridScope>(L, bc);
+    residual_restrict(L, bc);
 }
 // The FP32 cycle's residual + restriction in double-float arithmetic on FP32
 // pipes: coefficients as hi + lo pairs, b with its lo part on level 0 (blo,
@@ -294,7 +297,7 @@ template <class T>
 __global__ void k_prolong_gs1(Lvl<T> L, const T* xc, const CgState* st) {
     pdl_enter();
     if (st && st->done) return;
-    prolong_gs1<GridScope>(L, xc);
+    prolong_gs1(L, xc);
 }
 
 // The same level operations for an even side, one thread per 2 x 2 aggregate:
@@ -1081,9 +1084,9 @@ __global__ void __launch_bounds__(128) k_tail_matvec(const T* __restrict__ M, in
     }
 }
 
-// Fused visit kernels (fused.cuh): 16 x 32 tiles with 256 threads on large
-// levels; 8 x 16 tiles with 128 threads where a level has few cells, so that
-// small levels spread over more SMs and each thread stages less.
+// Fused visit kernels (fused.cuh): 16 x 32 tiles on large levels, 8 x 16 tiles
+// where a level has few cells, so that small levels spread over more SMs and
+// each thread stages less.
 constexpr int kMaxTileGrid = kMaxBlocks;
 
 template <int TH, int TW>
@@ -1267,8 +1270,8 @@ int num_levels_for(int n) {
 }
 
 size_t block_arena_bytes(int n, bool mixed, size_t sbudget) {
-    return mixed ? carve<float>(n, nullptr, nullptr, sbudget, nullptr).global_bytes
-                 : carve<double>(n, nullptr, nullptr, sbudget, nullptr).global_bytes;
+    return mixed ? carve<float>(n, nullptr, nullptr, sbudget, nullptr)
+                 : carve<double>(n, nullptr, nullptr, sbudget, nullptr);
 }
 
 size_t block_arena_stride(const int* sides, int64_t count, bool mixed, size_t sbudget) {

@@ -112,7 +112,7 @@ extern "C" int dgpu_apply_preconditioner_noalloc(const double* d_a, const double
         set_last_error("cycle_index must be 1 or 2");
         return DGPU_INVALID_INPUT;
     }
-    const size_t need = carve<double>((int)n, nullptr, nullptr, 0, nullptr).global_bytes;
+    const size_t need = carve<double>((int)n, nullptr, nullptr, 0, nullptr);
     if (need > kStatusOffset) {  // cannot happen for n <= kNoAllocMaxSide; kept as the invariant
         set_last_error("allocation-free scratch too small for this grid");
         return DGPU_INVALID_INPUT;

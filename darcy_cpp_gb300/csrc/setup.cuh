@@ -100,11 +100,10 @@ __device__ __forceinline__ void coarsen(const Lvl64& F, const Lvl64& C) {
 // FP32 copy of a level's coefficients for the mixed-precision cycle. When
 // the lo pointers are given, also the rounding remainders of e, nf, d
 // (c - (double)(float)c, rounded to FP32): hi + lo carries ~48 bits.
-template <class S>
 __device__ __forceinline__ void to_fp32(const Lvl64& L, float* e, float* nf, float* d, float* id, float* elo,
                                         float* nlo, float* dlo) {
     const int64_t m = (int64_t)L.n * L.n;
-    for (int64_t k = S::start(); k < m; k += S::stride()) {
+    for (int64_t k = GridScope::start(); k < m; k += GridScope::stride()) {
         float eh, el, nh, nl, dh, dl;  // split_f64: the conversions' bits without the FP64 pipe
         split_f64(L.e[k], eh, el);
         split_f64(L.nf[k], nh, nl);

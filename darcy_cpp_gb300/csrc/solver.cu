@@ -259,8 +259,6 @@ struct dgpu_context {
     std::string device_name;
     bool tune_loaded = false;
     std::map<std::string, BlockConfigPOD> tuned;
-    int last_block_threads = 0;
-    size_t last_block_smem = 0;
     // concurrent grid-engine solves: one stream, event pair and plan per slot
     std::vector<cudaStream_t> slot_streams;
     std::vector<cudaEvent_t> slot_events;
@@ -1092,18 +1090,20 @@ void save_tuning(dgpu_context* C) {
     std::fclose(fp);
 }
 
-// Shared memory for the batched engine's coarse levels and dense tail: sized
-// so that a 64^2 problem keeps levels 32^2 and 16^2 and its 64 x 64 tail on
-// chip with two CTAs per SM.
+// Shared memory for the batched engine's dense tail and levels, from the
+// coarsest up (carve in block.cuh). What a budget holds of a 64^2 problem: the
+// tail takes 20 KiB in FP32 and 36 in FP64, with the levels 8^2 and 16^2 27 and
+// 50, with 32^2 51 and 98, level 0 in FP32 148 (its iterate up to 68). So the
+// default, 48 KiB (FP32) and 96 KiB (FP64), is the tail and every level but 0,
+// except the diagonal of 32^2.
 size_t smem_budget_for(bool mixed) { return mixed ? 48 * 1024 : 96 * 1024; }
-// A budget large enough for the whole FP32 cycle of a 64^2 problem (every
-// level and the tail on chip, one CTA per SM): then only the FP64 CG vectors
-// and fine-level coefficients live in global memory.
+// The whole FP32 cycle of a 64^2 problem, one CTA per SM: then only the FP64 CG
+// vectors and fine-level coefficients live in global memory. (Device ms at the
+// best of 256 to 1024 threads: 4096 x 64^2 mixed 20.3 with this budget, 13.5
+// with the next, 12.4 with 32 KiB; 512 x 128^2 mixed 18.9, 18.9, 18.0 with 48.)
 constexpr size_t kSmemBudgetLarge = 180 * 1024;
-// Level 0 of a 64^2 FP32 cycle alone (6 x 16 KiB), two CTAs of up to 512
-// threads per SM: the cycle's heaviest level on chip, and the FP64 CG vectors
-// and coefficients of the two resident problems per SM (~300 KB each) within
-// the L2.
+// The same without two or three of level 0's six arrays, two CTAs of up to 512
+// threads per SM.
 constexpr size_t kSmemBudgetLevel0 = 100 * 1024;
 
 // Autotuning key of a batch (loads the tuning file on first use). Batches
@@ -1343,8 +1343,6 @@ void block_solve(dgpu_context* C, int64_t count, const std::vector<int>& sides, 
         C->tuned[key] = BlockConfigPOD{cfg.threads, cfg.smem, false};
         save_tuning(C);
     }
-    C->last_block_threads = cfg.threads;
-    C->last_block_smem = cfg.smem;
 
     CK(cudaEventRecord(C->ev0, s));
     if (pipelined) {
