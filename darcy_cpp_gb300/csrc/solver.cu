@@ -1213,9 +1213,13 @@ void block_solve(dgpu_context* C, int64_t count, const std::vector<int>& sides, 
     CK(cudaMemcpyAsync((void*)A.side, sides.data(), sizeof(int) * count, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync((void*)A.off, off.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
 
-    std::vector<int> distinct = sides;  // what the arenas are sized for
-    std::sort(distinct.begin(), distinct.end());
-    distinct.erase(std::unique(distinct.begin(), distinct.end()), distinct.end());
+    std::vector<int> distinct;  // the sides that the arenas are sized for
+    std::vector<char> seen((size_t)maxside + 1, 0);
+    for (int n : sides)
+        if (!seen[(size_t)n]) {
+            seen[(size_t)n] = 1;
+            distinct.push_back(n);
+        }
     // launch with a given shape over `n_prob` entries of `order` from `first`
     // (slot 1: the second compute stream, its own arenas and work counter)
     auto launch = [&](const BlockConfig& cfg, int64_t n_prob, int64_t first = 0, int slot = 0) {
