@@ -132,10 +132,12 @@ std::vector<double> make_x0(const py::object& x0, const std::vector<int64_t>& sh
 class Packed {
 public:
     void allocate(size_t total) { out_.reset(new double[total]); }
-    void add(const Array& arr, bool converted = false) {
-        keep_.push_back(arr);
+    void add(const double* src, size_t len) { pieces_.push_back(Piece{src, 0.0, len}); }  // the caller keeps src
+    void add(Array&& arr, bool converted) {
         pieces_.push_back(Piece{arr.data(), 0.0, (size_t)arr.size()});
-        if (converted && (converted_ += (size_t)arr.nbytes()) >= kConverted) flush();
+        converted_ += converted ? (size_t)arr.nbytes() : 0;
+        keep_.push_back(std::move(arr));
+        if (converted_ >= kConverted) flush();
     }
     void add(double value, size_t len) { pieces_.push_back(Piece{nullptr, value, len}); }
     void flush() {
@@ -325,20 +327,23 @@ PYBIND11_MODULE(_core, m) {
             if (!x0.is_none()) u0packed.allocate(total);
             for (int64_t q = 0; q < count; ++q) {
                 const int64_t n = sides[q];
-                packed.add(keep[(size_t)q]);
+                packed.add(keep[(size_t)q].data(), (size_t)(n * n));
                 if (f_list) {
                     const py::object fq = py::list(f)[q];
                     double value;
                     Array arr;
-                    if (rhs_array(fq, n, value, arr))
-                        fpacked.add(arr, arr.ptr() != fq.ptr());
-                    else
+                    if (rhs_array(fq, n, value, arr)) {
+                        const bool converted = arr.ptr() != fq.ptr();
+                        fpacked.add(std::move(arr), converted);
+                    } else {
                         fpacked.add(value, (size_t)(n * n));
+                    }
                 }
                 if (!x0.is_none()) {
                     const py::object xq = x0l[q];
-                    const Array arr = x0_array(xq, {n, n});
-                    u0packed.add(arr, arr.ptr() != xq.ptr());
+                    Array arr = x0_array(xq, {n, n});
+                    const bool converted = arr.ptr() != xq.ptr();
+                    u0packed.add(std::move(arr), converted);
                 }
             }
             packed.flush();
