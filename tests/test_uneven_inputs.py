@@ -45,7 +45,7 @@ def test_fields_written_by_another_thread_are_seen_whole() -> None:
     between. Tolerance: launch shapes differ, so sums round differently."""
     import darcy_cpp_gb300 as darcy
 
-    n, count = 256, 200  # 105 MB: packed by several threads
+    n, count = 256, 150  # 79 MB, packed by several threads; too few problems for the shape tuner
     ones = np.ones((n, n))
     u1 = darcy.solve_batch_uneven([ones], max_iter=1).u[0]
     fields = [ones.copy() for _ in range(count)]
